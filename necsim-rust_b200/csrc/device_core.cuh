@@ -28,21 +28,62 @@ constexpr uint64_t kInvPhi = 0x9e3779b97f4a7c15ULL;
 // core::f64::consts::TAU
 constexpr double kTau = 6.283185307179586;
 
+// The 128-bit product of two 64-bit words from four 32 x 32 -> 64 products
+// (separate low and high product instructions would take seven).
+__device__ __forceinline__ uint64_t mul_wide(uint32_t a, uint32_t b) { return (uint64_t)a * (uint64_t)b; }
+__device__ __forceinline__ void mul_64_64(uint64_t a, uint64_t b, uint64_t &lo, uint64_t &hi) {
+    const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
+    const uint64_t p00 = mul_wide(a0, b0), p01 = mul_wide(a0, b1), p10 = mul_wide(a1, b0), p11 = mul_wide(a1, b1);
+    uint32_t l1, h0, h1;
+    asm("{\n\t.reg .u32 t1, t2, t3;\n\t"
+        "add.cc.u32 t1, %3, %4;\n\t"
+        "addc.cc.u32 t2, %5, %6;\n\t"
+        "addc.u32 t3, %7, 0;\n\t"
+        "add.cc.u32 %0, t1, %8;\n\t"
+        "addc.cc.u32 %1, t2, %9;\n\t"
+        "addc.u32 %2, t3, 0;\n\t}"
+        : "=r"(l1), "=r"(h0), "=r"(h1)
+        : "r"((uint32_t)(p00 >> 32)), "r"((uint32_t)p01), "r"((uint32_t)(p01 >> 32)), "r"((uint32_t)p11),
+          "r"((uint32_t)(p11 >> 32)), "r"((uint32_t)p10), "r"((uint32_t)(p10 >> 32)));
+    lo = ((uint64_t)l1 << 32) | (uint32_t)p00;
+    hi = ((uint64_t)h1 << 32) | h0;
+}
+
 // wyhash.rs:85-96: 64x64 -> 128 multiply, low and high halves xor-folded
 __device__ __forceinline__ uint64_t wymum(uint64_t a, uint64_t b) {
-    const uint64_t lo = a * b;
-    const uint64_t hi = __umul64hi(a, b);
+    uint64_t lo, hi;
+    mul_64_64(a, b, lo, hi);
     return (a ^ lo) ^ (b ^ hi);
 }
 
-// wyhash.rs:99-119
-__device__ __forceinline__ uint64_t seahash_diffuse(uint64_t x) {
-    x *= kSeaHashK;
+// The diffusion after its first multiplication.
+__device__ __forceinline__ uint64_t seahash_finish(uint64_t x) {
     const uint64_t a = x >> 32;
     const uint64_t b = x >> 60;
     x ^= a >> b;
     x *= kSeaHashK;
     return x;
+}
+
+// wyhash.rs:99-119
+__device__ __forceinline__ uint64_t seahash_diffuse(uint64_t x) { return seahash_finish(x * kSeaHashK); }
+
+// The inverse of an odd constant modulo 2^64 (Newton's iteration doubles the
+// correct low bits, three at the start).
+constexpr uint64_t inverse_mod_2_64(uint64_t a) {
+    uint64_t x = a;
+    for (int j = 0; j < 6; ++j) x *= 2 - a * x;
+    return x;
+}
+constexpr uint64_t kSeaHashKInverse = inverse_mod_2_64(kSeaHashK);
+static_assert(kSeaHashK * kSeaHashKInverse == 1, "not an inverse");
+
+// The input of a diffusion: the xor changes only the low word, by a value
+// that the unchanged high word determines.
+__device__ __forceinline__ uint64_t seahash_undiffuse(uint64_t x) {
+    x *= kSeaHashKInverse;
+    x ^= (x >> 32) >> (x >> 60);
+    return x * kSeaHashKInverse;
 }
 
 __device__ __forceinline__ uint64_t swap_halves(uint64_t v) { return (v << 32) | (v >> 32); }
@@ -87,16 +128,24 @@ __device__ __forceinline__ uint64_t location_term(uint64_t seed, uint64_t locati
     return swap_halves(seahash_diffuse(location_index)) ^ (seed ^ kWyP0);
 }
 
+// WyHash state after prime_with(location, time_index), from the location
+// term and time_index * K (K the diffusion's multiplier)
+__device__ __forceinline__ uint64_t primed_state_k(uint64_t loc_term, uint64_t time_index_k) {
+    const uint64_t h = wymum(loc_term, swap_halves(seahash_finish(time_index_k)) ^ kWyP2);
+    return wymum(h, 16ULL ^ kWyP5);
+}
+
 // WyHash state after prime_with(location, time_index), from the location term
 __device__ __forceinline__ uint64_t primed_state(uint64_t loc_term, uint64_t time_index) {
-    const uint64_t h = wymum(loc_term, swap_halves(seahash_diffuse(time_index)) ^ kWyP2);
-    return wymum(h, 16ULL ^ kWyP5);
+    return primed_state_k(loc_term, time_index * kSeaHashK);
 }
 
 // the k-th sample_u64 after priming to s0
 __device__ __forceinline__ uint64_t draw_at(uint64_t s0, uint32_t k) {
     const uint64_t s = s0 + (uint64_t)k * kWyP0;
-    return seahash_diffuse(wymum(s ^ kWyP1, s));
+    uint64_t lo, hi;
+    mul_64_64(s ^ kWyP1, s, lo, hi);
+    return seahash_diffuse(lo ^ hi ^ kWyP1);  // wymum(s ^ P1, s): its factors' xor is P1
 }
 
 __device__ __forceinline__ double unit_closed_open(uint64_t v) {
@@ -105,6 +154,26 @@ __device__ __forceinline__ double unit_closed_open(uint64_t v) {
 __device__ __forceinline__ double unit_open_closed(uint64_t v) {
     return __dmul_rn(__ull2double_rn((v >> 11) + 1ULL), 0x1.0p-53);
 }
+
+// The 53-bit integer d >> 11 of a sample as an exact double: its low 32 and
+// high 21 bits are placed in the mantissas of 2^52 and 2^84, and two exact
+// additions remove the offsets.  A conversion instruction takes as long (28
+// against 30 cycles in a dependent chain on a B200) but holds its pipe for
+// 12.5 cycles per warp, the two additions for 4.
+__device__ __forceinline__ double sample_bits(uint64_t d) {
+    const uint32_t lo = __funnelshift_r((uint32_t)d, (uint32_t)(d >> 32), 11), hi = (uint32_t)(d >> 43);
+    const double h = __hiloint2double(0x45300000, (int)hi), l = __hiloint2double(0x43300000, (int)lo);
+    return __dadd_rn(__dsub_rn(h, 0x1.00000001p84), l);  // (2^84 + hi 2^32) - (2^84 + 2^52) + (2^52 + lo)
+}
+
+// An integer below 2^51 as an exact double.
+__device__ __forceinline__ double exact_double(uint64_t v) {
+    return __dsub_rn(__longlong_as_double((long long)(v | 0x4330000000000000ULL)), 0x1p52);
+}
+
+// floor(v) of 0 <= v < 2^32: adding 2^52 rounded towards zero leaves it in
+// the low mantissa word (30 cycles in a chain; floor and a conversion take 78).
+__device__ __forceinline__ uint32_t floor_u32(double v) { return (uint32_t)__double2loint(__dadd_rz(v, 0x1p52)); }
 
 // Rust `f64 as u64` for the non-negative finite values these call sites see
 // (floor of a product of a unit sample and a table length, or of t / dt);
@@ -360,14 +429,24 @@ __device__ __forceinline__ uint32_t coalescence_index(uint64_t d, uint32_t habit
     return f64_to_u32(floor(__dmul_rn(unit_closed_open(d), __uint2double_rn(habitat))));
 }
 
-// habitat/almost_infinite.rs:100-114 clamp_round_dispersal
+// One coordinate of clamp_round_dispersal (habitat/almost_infinite.rs:
+// 100-114): x + round(v) modulo 2^32, where `round` rounds halves away from
+// zero and the conversion to i64 saturates (NaN -> 0).  Both of the
+// reference's remainders by 2^32 keep the low word of the wrapping 64-bit
+// sum.  Below 2^51 the integer part is read from the mantissa of |v| + 2^52
+// (rounded towards zero) and the fraction, exact, is compared with 1/2.
+__device__ __forceinline__ uint32_t round_onto_plane(uint32_t x, double v) {
+    const double m = fabs(v);
+    if (!(m < 0x1p51)) return x + (uint32_t)(uint64_t)f64_to_i64(round(v));
+    const double t = __dadd_rz(m, 0x1p52);
+    const uint32_t n = (uint32_t)__double2loint(t) + (__dsub_rn(m, __dsub_rn(t, 0x1p52)) >= 0.5 ? 1u : 0u);
+    return v < 0.0 ? x - n : x + n;
+}
+
 __device__ __forceinline__ void clamp_round_dispersal(uint32_t x, uint32_t y, double dx, double dy,
                                                       uint32_t &tx, uint32_t &ty) {
-    const int64_t wrap = (int64_t)1 << 32;
-    const int64_t nx = ((int64_t)x + f64_to_i64(round(dx))) % wrap;
-    const int64_t ny = ((int64_t)y + f64_to_i64(round(dy))) % wrap;
-    tx = (uint32_t)((nx + wrap) % wrap);
-    ty = (uint32_t)((ny + wrap) % wrap);
+    tx = round_onto_plane(x, dx);
+    ty = round_onto_plane(y, dy);
 }
 
 // almost_infinite_clark2dt.rs:96-107 with clark2dt::cdf_inverse and

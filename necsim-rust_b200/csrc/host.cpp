@@ -486,6 +486,25 @@ PoissonConsts make_poisson_consts(double lambda, double delta_t) {
     return c;
 }
 
+// Whether the kernels' chain_run may step the scenario's lineages: each
+// community has fewer than 2^32 cells, and a SpatiallyImplicit location is
+// in one community only (the metacommunity lies at the plane's far corner;
+// where it reaches into the local extent, the reference tests local first).
+bool chain_scenario(const SimParams &p, int32_t kind) {
+    const uint64_t most = 0xffffffffULL;
+    // a power of two whose products with event times stay normal
+    if (p.inv_delta_t == 0.0 || !(p.delta_t > 0x1p-256 && p.delta_t < 0x1p256)) return false;
+    switch (kind) {
+    case NECSIM_NON_SPATIAL: return (uint64_t)p.width * p.height <= most;
+    case NECSIM_SPATIALLY_IMPLICIT:
+        return (uint64_t)p.width * p.height <= most && (uint64_t)p.meta_width * p.meta_height <= most &&
+               (p.meta_ox > p.width - 1 || p.meta_oy > p.height - 1);
+    case NECSIM_ALMOST_INFINITE_NORMAL:
+    case NECSIM_ALMOST_INFINITE_CLARK2DT: return true;
+    default: return false;
+    }
+}
+
 SimParams base_params(const necsim_scenario &sc, const necsim_args &args, uint64_t wy_seed) {
     SimParams p;
     std::memset(&p, 0, sizeof(p));
@@ -539,6 +558,7 @@ SimParams base_params(const necsim_scenario &sc, const necsim_args &args, uint64
         p.clark_exponent = 1.0 / sc.tail_p;
     }
     if (sc.kind == NECSIM_WRAPPING_NOISE) p.noise = noise_habitat(sc);
+    p.chain = chain_scenario(p, sc.kind) ? 1 : 0;
     p.pause_before = -1.0;
     return p;
 }

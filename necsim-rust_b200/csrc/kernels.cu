@@ -809,6 +809,383 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
     }
 }
 
+// ---- the cooperative step of the scenarios without tables ----
+//
+// chain_run is coop_run for NonSpatial, SpatiallyImplicit and AlmostInfinite
+// (the same lane roles, the same results), written for the latency of the
+// one dependent chain that every tail is:
+//  * the lineage is its location term, its time bucket and its last event
+//    time in units of delta_t (a power of two: every product with it is
+//    exact); its coordinates are recovered from the location term when it
+//    stops (location_term is invertible), so an event moves two words
+//    between lanes where eight moved before, and a target needs no division
+//    (its injection is cell * deme + index);
+//  * a lane's search result and the candidate lane that holds its event are
+//    one 32-bit key, so one warp minimum selects both (the candidate's lane
+//    is looked up in the bucket's own packed table);
+//  * the time index of the next prime is kept multiplied by the diffusion's
+//    constant, so a selection adds (buckets advanced) * constant to it;
+//  * samples become doubles by mantissa placement, products are rounded
+//    towards zero into integers, and a bucket looks at the two or three
+//    events whose samples are drawn anyway; a bucket with more events (found
+//    from one more threshold) is resolved by the whole warp;
+//  * the loop over events holds only what every event needs: a lone warp
+//    waits for instructions when the loop outgrows the instruction cache.
+//    Speciations, horizons, migrations and the rarer selections leave it
+//    with the event computed.
+// Measured with one lineage on a B200 (1,965 MHz), coop_run -> chain_run:
+// NonSpatial 1,772 -> 673 cycles per event, SpatiallyImplicit 1,747 -> 663,
+// AlmostInfinite Normal 2,793 -> 1,892, Clark2Dt 3,376 -> 2,568.  The bound
+// is the instruction count: a lone warp issues one instruction every two
+// cycles, and NonSpatial takes 329 per event (48 a prime, 31 a sample).
+template <int KIND>
+constexpr bool kChainKind = KIND == kNonSpatial || KIND == kSpatiallyImplicit || KIND == kAlmostInfiniteNormal;
+
+// Whether chain_run takes the simulation's round: SimParams.chain (delta_t a
+// power of two, every table length below 2^32, no metacommunity cell inside
+// the local community) and time buckets that are exact doubles.
+template <int KIND>
+__device__ __forceinline__ bool chain_takes(const SimParams &p, const Lane &l) {
+    const double most = __dmul_rn(p.delta_t, 0x1p50);
+    return kChainKind<KIND> && p.chain != 0 && l.horizon < most && l.last < most && p.min_event_time < most;
+}
+
+// A bucket lane's search result, one word that orders by bucket: buckets
+// advanced << 28 (the event's own time bucket: one more than its bucket when
+// start + u rounds up), the bucket << 20, flags, the event's index << 8 and
+// the lane of its candidate.  A shuffle reads the low five bits of its lane
+// operand only, so the word, and the word >> 20, name a lane as they are.
+constexpr uint32_t kSelMore = 1u << 19;         // the bucket has events beyond the samples drawn
+constexpr uint32_t kSelStop = 1u << 18;         // the event is at or beyond the horizon
+constexpr uint32_t kNoCandidate = 0xe0u;        // the event is not among the candidates
+constexpr uint32_t kSelNone = 0xffffffffu;      // no event in the eight buckets
+constexpr uint32_t kSelLeave = kSelMore | kSelStop | kNoCandidate;
+constexpr uint32_t kAttention = 0xffffffffu;    // high word of a candidate's location term: leave the loop
+constexpr double kNeverTime = 0x1p1000;         // no event
+
+// candidate lanes of bucket b's events 0..3, one byte each
+constexpr uint32_t coop_lanes_of(unsigned b) {
+    uint32_t w = kNoCandidate * 0x01010101u;
+    for (int j = 0; j < 32 - (int)kCoopBuckets; ++j)
+        if (kCoopPairList[j].b == b && kCoopPairList[j].k < 4)
+            w = (w & ~(0xffu << (8 * kCoopPairList[j].k))) | ((kCoopBuckets + j) << (8 * kCoopPairList[j].k));
+    return w;
+}
+constexpr uint32_t kCoopLanes0 = coop_lanes_of(0), kCoopLanes1 = coop_lanes_of(1), kCoopLanes2 = coop_lanes_of(2),
+                   kCoopLanes3 = coop_lanes_of(3), kCoopLanes4 = coop_lanes_of(4), kCoopLanes5 = coop_lanes_of(5),
+                   kCoopLanes6 = coop_lanes_of(6), kCoopLanes7 = coop_lanes_of(7);
+__device__ __forceinline__ uint32_t coop_lane_table(unsigned b) {
+    const uint32_t lo = b < 2u ? (b ? kCoopLanes1 : kCoopLanes0) : (b == 2u ? kCoopLanes2 : kCoopLanes3);
+    const uint32_t hi = b < 6u ? (b == 5u ? kCoopLanes5 : kCoopLanes4) : (b == 6u ? kCoopLanes6 : kCoopLanes7);
+    return b < 4u ? lo : hi;
+}
+
+// A community's extent (NonSpatial, or one of SpatiallyImplicit's two).
+struct Community {
+    uint32_t ox, oy, width, deme;
+    uint64_t cells;
+};
+template <int KIND>
+__device__ __forceinline__ Community community_of(const SimParams &p, bool local) {
+    if (KIND == kSpatiallyImplicit && !local)
+        return {p.meta_ox, p.meta_oy, p.meta_width, p.meta_deme, (uint64_t)p.meta_width * p.meta_height};
+    return {0u, 0u, p.width, p.deme, (uint64_t)p.width * p.height};
+}
+
+// The coordinates of a location term (the inverse of location_term and
+// injection_at).
+template <int KIND>
+__device__ __forceinline__ void chain_unpack(const SimParams &p, uint64_t loc_term, bool local, uint32_t &x,
+                                             uint32_t &y, uint32_t &i) {
+    const uint64_t inj = seahash_undiffuse(swap_halves(loc_term ^ (p.seed ^ kWyP0)));
+    if (KIND == kAlmostInfiniteNormal) {
+        x = (uint32_t)inj;
+        y = (uint32_t)(inj >> 32);
+        i = 0;
+        return;
+    }
+    const Community c = community_of<KIND>(p, local);
+    const uint64_t cell = inj / c.deme;
+    i = (uint32_t)(inj - cell * c.deme);
+    const uint32_t row = (uint32_t)cell / c.width;
+    x = c.ox + ((uint32_t)cell - row * c.width);
+    y = c.oy + row;
+}
+
+// A lineage between the events of chain_run.
+struct Chain {
+    uint64_t loc_term;
+    uint64_t base;       // time bucket the search starts in
+    uint64_t reprime;    // of a peeked event
+    double before;       // the search's start, in units of delta_t
+    double next;         // peeked event time, in units of delta_t
+    uint32_t x, y;       // AlmostInfinite
+    uint32_t moved;      // events executed
+    bool peek;           // `next` and `reprime` hold a peeked event
+    bool local;          // SpatiallyImplicit: in the local community
+};
+
+// Events of a lineage in one community (LOCAL: SpatiallyImplicit's local
+// one, which it leaves by migration: kStepMoved) until it stops
+// (kStepStop, with the peek) or speciates (kStepSpeciated, at c.next).
+template <int KIND, bool LOCAL>
+__device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p, const EventSink &k,
+                                           const volatile unsigned *stop) {
+    constexpr bool kMigrates = KIND == kSpatiallyImplicit && LOCAL;
+    const unsigned lane = threadIdx.x & 31u;
+    const bool bucket_lane = lane < kCoopBuckets;
+    uint32_t my_b = lane, my_k = 0;
+    if (!bucket_lane) {
+        const unsigned j = lane - kCoopBuckets;
+        const uint64_t w = j < 8u ? kCoopPairWord0 : (j < 16u ? kCoopPairWord1 : kCoopPairWord2);
+        const uint32_t pr = (uint32_t)(w >> (8u * (j & 7u))) & 0xffu;
+        my_b = pr & 15u;
+        my_k = pr >> 4;
+    }
+    const uint64_t my_tadd_k = ((uint64_t)my_b + (bucket_lane ? 0ULL : kInvPhi * (uint64_t)(my_k + 1u))) * kSeaHashK;
+    // the keys of this bucket's events 0..2 (no candidate lane finds one)
+    const uint32_t lanes_b = coop_lane_table(my_b & 7u);
+    const uint32_t key_b = (my_b << 28) | (my_b << 20);
+    const uint32_t key0 = key_b | (lanes_b & 0xffu), key1 = key_b | (1u << 8) | ((lanes_b >> 8) & 0xffu),
+                   key2 = key_b | (2u << 8) | ((lanes_b >> 16) & 0xffu);
+    const uint64_t seed_term = p.seed ^ kWyP0;
+    // X > t  <=>  d > t 2^11 + 2047 for X = d >> 11 (never for t >= 2^53 - 1)
+    auto above = [](uint64_t t) { return t >= (1ULL << 53) - 1 ? ~0ULL : (t << 11) | 2047ULL; };
+    const uint64_t more0 = above(p.pois.threshold[0]), more1 = above(p.pois.threshold[1]),
+                   more2 = above(p.pois.threshold[2]), more3 = above(p.pois.threshold[3]);
+    // X < t  <=>  d <= t 2^11 - 1 for 0 < t <= 2^53
+    const uint64_t leave_at_most = ((kMigrates ? p.migration_threshold : p.nu_threshold) << 11) - 1ULL;
+    // floor(u L) = floor(X (L 2^-53)): the scaling is exact, so the product
+    // rounds like the reference's; below 2^32 it never rounds up to L (L and
+    // its predecessor are further apart than half of L 2^-53), so the
+    // reference's clamp to L - 1 changes nothing
+    const Community com = community_of<KIND>(p, LOCAL);
+    const double cells_u = __dmul_rn(__ull2double_rn(com.cells), 0x1p-53);
+    const double deme_u = __dmul_rn(__uint2double_rn(com.deme), 0x1p-53);
+    const uint64_t deme_k = (uint64_t)com.deme * kSeaHashK;
+    const double sigma = p.sigma, horizon = __dmul_rn(l.horizon, p.inv_delta_t);
+    const bool clark = p.clark != 0;
+
+    constexpr uint32_t kFlush = 1u << 30;  // `moved` is added up before it overflows
+    uint64_t tk = 0, start_bits = 0;
+    // the event count at which the inner loop is left: to look at `stop`, for
+    // a peeked event, and at every event when dispersal events are reported
+    uint32_t attend = 0;
+    auto enter = [&] {
+        tk = c.peek ? c.reprime * kSeaHashK : c.base * kSeaHashK + my_tadd_k;
+        start_bits = 0x4330000000000000ULL | (c.base + my_b);
+        attend = c.peek || k.report_dispersal ? c.moved : (stop ? (c.moved + 31u) & ~31u : kFlush);
+    };
+    enter();
+    for (;;) {
+        uint64_t s, d1, loc_next;
+        uint32_t sel, tx = 0, ty = 0;
+        double mine;
+        bool leave;
+        for (;;) {
+            // a peeked event is computed by every lane, a search by the lanes' roles
+            s = primed_state_k(c.loc_term, tk);
+            d1 = draw_at(s, 1);
+            const uint64_t d2 = draw_at(s, 2), d3 = draw_at(s, 3), d4 = draw_at(s, 4);
+            const double v2 = sample_bits(d2), v3 = sample_bits(d3), v4 = sample_bits(d4);
+
+            // candidate view: the event that this lane's samples make
+            // (event_sampler/independent.rs:112-222); a local lineage never
+            // speciates and draws a migration test before its target
+            // (dispersal_sampler/spatially_implicit.rs:58-86)
+            leave = (kMigrates ? d2 : d1) <= leave_at_most;
+            uint64_t inj_k;
+            if constexpr (KIND == kAlmostInfiniteNormal) {
+                if (clark)
+                    clark2dt_dispersal_draw(d2, d3, p.clark_shape_u, p.clark_exponent, c.x, c.y, tx, ty);
+                else
+                    normal_dispersal_draw(d2, d3, sigma, c.x, c.y, tx, ty);
+                inj_k = (((uint64_t)ty << 32) | (uint64_t)tx) * kSeaHashK;
+            } else {
+                const uint32_t cell = floor_u32(__dmul_rn(kMigrates ? v3 : v2, cells_u));
+                const uint32_t i = floor_u32(__dmul_rn(kMigrates ? v4 : v3, deme_u));
+                inj_k = (uint64_t)cell * deme_k + (uint64_t)i * kSeaHashK;
+            }
+            loc_next = swap_halves(seahash_finish(inj_k)) ^ seed_term;
+            const uint32_t next_hi = leave ? kAttention : (uint32_t)(loc_next >> 32);
+
+            // bucket view: the earliest event of this lane's bucket after
+            // `before` among its first three (ties: lowest index),
+            // poisson.rs:48-100
+            const double start = __dsub_rn(__longlong_as_double((long long)start_bits), 0x1p52);
+            const double q0 = __fma_rn(v2, 0x1p-53, start);  // start + u: u is exact
+            const double q1 = __fma_rn(v3, 0x1p-53, start);
+            const double q2 = __fma_rn(v4, 0x1p-53, start);
+            mine = d1 > more0 && q0 > c.before ? q0 : kNeverTime;
+            uint32_t key = key0;
+            if (d1 > more1 && q1 > c.before && q1 < mine) {
+                mine = q1;
+                key = key1;
+            }
+            if (d1 > more2 && q2 > c.before && q2 < mine) {
+                mine = q2;
+                key = key2;
+            }
+            if (mine >= __dadd_rn(start, 1.0)) key += 1u << 28;  // rounded up (or none)
+            if (mine >= horizon) key |= kSelStop;
+            const bool more = d1 > more3;
+            if (more) key |= kSelMore;
+            const bool found = bucket_lane && (more || mine < kNeverTime);
+            sel = __reduce_min_sync(kFull, found ? key : kSelNone);
+
+            const double q = __shfl_sync(kFull, mine, (int)(sel >> 20));
+            const uint32_t lo = __shfl_sync(kFull, (uint32_t)loc_next, (int)sel);
+            const uint32_t hi = __shfl_sync(kFull, next_hi, (int)sel);
+            if ((sel & kSelLeave) != 0u || hi == kAttention || c.moved == attend) break;
+            if (KIND == kAlmostInfiniteNormal) {
+                c.x = __shfl_sync(kFull, tx, (int)sel);
+                c.y = __shfl_sync(kFull, ty, (int)sel);
+            }
+            c.loc_term = ((uint64_t)hi << 32) | lo;
+            tk += (uint64_t)(sel >> 28) * kSeaHashK;
+            start_bits += sel >> 28;
+            c.before = q;
+            c.moved += 1;
+        }
+
+        const bool searched = !c.peek;
+        uint32_t cand = lane;
+        if (searched) {
+            c.base = (start_bits & 0xfffffffffffffULL) - my_b;
+            if (sel == kSelNone) {  // eight empty buckets: the next eight
+                c.base += kCoopBuckets;
+                enter();
+                continue;
+            }
+            const uint32_t b_sel = (sel >> 20) & 31u;
+            uint32_t k_sel = (sel >> 8) & 0xffu;
+            cand = sel & 0xffu;
+            double q = __shfl_sync(kFull, mine, (int)b_sel);
+            if (sel & kSelMore) {
+                // the bucket has more than three events (3% of the buckets
+                // with events at lambda delta_t = 1): lane j draws j, j + 32, ...
+                const uint64_t s_b = __shfl_sync(kFull, s, (int)b_sel), d1_b = __shfl_sync(kFull, d1, (int)b_sel);
+                const double start_b = exact_double(c.base + b_sel);
+                const uint32_t n_ev = poisson_count(d1_b, p.pois);
+                long long best = kNoEvent;
+                uint32_t best_k = 0xffffffffu;
+                for (uint32_t j = lane; j < n_ev; j += 32u) {
+                    const long long eb = event_time_bits(start_b, draw_at(s_b, j + 2u), 1.0);
+                    if (eb > __double_as_longlong(c.before) && eb < best) {
+                        best = eb;
+                        best_k = j;
+                    }
+                }
+                const uint32_t hi = __reduce_min_sync(kFull, (uint32_t)(best >> 32));
+                const bool in_hi = (uint32_t)(best >> 32) == hi;
+                const uint32_t lo = __reduce_min_sync(kFull, in_hi ? (uint32_t)best : 0xffffffffu);
+                k_sel = __reduce_min_sync(kFull, in_hi && (uint32_t)best == lo ? best_k : 0xffffffffu);
+                if (k_sel == 0xffffffffu) {  // all of them at or before `before`
+                    c.base += b_sel + 1u;
+                    enter();
+                    continue;
+                }
+                q = __hiloint2double((int)hi, (int)lo);
+                const uint32_t lanes_sel = __shfl_sync(kFull, lanes_b, (int)b_sel);
+                cand = k_sel < 4u ? (lanes_sel >> (8u * k_sel)) & 0xffu : kNoCandidate;
+            }
+            c.next = q;
+            c.reprime = c.base + b_sel + kInvPhi * (uint64_t)(k_sel + 1u);
+            // the reference's early stop `next_event_time >= level_time`
+            // (monolithic/mod.rs:228-239), or an interruption
+            bool keep = q >= horizon;
+            if (!keep && stop && c.moved == attend)
+                keep = __shfl_sync(kFull, lane == 0 ? *stop : 1u, 0) == 0u;
+            c.peek = keep || cand == kNoCandidate;
+            if (keep) return kStepStop;
+            if (c.peek) {  // not speculated: computed as a peeked event
+                enter();
+                continue;
+            }
+        } else if (c.next >= horizon) {
+            return kStepStop;
+        }
+        c.peek = false;
+        const bool leaves = __shfl_sync(kFull, leave ? 1 : 0, (int)cand) != 0;
+        if (leaves && !kMigrates) return kStepSpeciated;
+        if (k.report_dispersal && lane == 0) chain_unpack<KIND>(p, c.loc_term, LOCAL, l.x, l.y, l.i);
+        if (leaves) {
+            // migration: the target in the metacommunity from samples 3 and 4
+            const uint64_t s_e = __shfl_sync(kFull, s, (int)cand);
+            const Community meta = community_of<KIND>(p, false);
+            const uint32_t cell = floor_u32(__dmul_rn(sample_bits(draw_at(s_e, 3)),
+                                                      __dmul_rn(__ull2double_rn(meta.cells), 0x1p-53)));
+            const uint32_t i = floor_u32(__dmul_rn(sample_bits(draw_at(s_e, 4)),
+                                                   __dmul_rn(__uint2double_rn(meta.deme), 0x1p-53)));
+            c.loc_term = location_term(p.seed, (uint64_t)cell * meta.deme + i);
+        } else {
+            c.loc_term = __shfl_sync(kFull, loc_next, (int)cand);
+            c.x = __shfl_sync(kFull, tx, (int)cand);
+            c.y = __shfl_sync(kFull, ty, (int)cand);
+        }
+        if (k.report_dispersal && lane == 0) {
+            uint32_t ex, ey, ei;
+            chain_unpack<KIND>(p, c.loc_term, LOCAL && !leaves, ex, ey, ei);
+            l.next = __dmul_rn(c.next, p.delta_t);
+            emit_dispersal(l, k, ex, ey, ei);
+            l.last = l.next;
+        }
+        c.before = c.next;
+        c.base = f64_to_u64(floor(c.next));
+        c.moved += 1;
+        if (leaves) return kStepMoved;
+        if (c.moved >= kFlush) {
+            l.steps += c.moved;
+            c.moved = 0;
+        }
+        enter();
+    }
+}
+
+template <int KIND>
+__device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const EventSink &k, uint64_t &events,
+                                         const volatile unsigned *stop = nullptr) {
+    Chain c;
+    c.loc_term = location_term(p.seed, lane_injection<KIND>(l, p));
+    const double before = l.last > p.min_event_time ? l.last : p.min_event_time;
+    c.base = time_bucket(p, before);
+    c.before = __dmul_rn(before, p.inv_delta_t);
+    c.next = __dmul_rn(l.next, p.inv_delta_t);
+    c.reprime = l.reprime;
+    c.peek = l.has_next;
+    c.x = l.x;
+    c.y = l.y;
+    c.moved = 0;
+    c.local = KIND != kSpatiallyImplicit || in_local(p, l.x, l.y);
+    const uint64_t steps = l.steps;
+    int result = kStepMoved;
+    if (KIND == kSpatiallyImplicit && c.local) {
+        result = chain_phase<KIND, true>(c, l, p, k, stop);
+        c.local = result != kStepMoved;
+    }
+    if (result == kStepMoved) result = chain_phase<KIND, KIND != kSpatiallyImplicit>(c, l, p, k, stop);
+    l.steps += c.moved;
+    if (l.steps != steps) l.last = __dmul_rn(c.before, p.delta_t);
+    if (result == kStepSpeciated) l.steps += 1;
+    events += l.steps - steps;
+    l.next = __dmul_rn(c.next, p.delta_t);
+    l.reprime = c.reprime;
+    l.has_next = result == kStepStop;
+    chain_unpack<KIND>(p, c.loc_term, c.local, l.x, l.y, l.i);
+    if (result == kStepSpeciated && (threadIdx.x & 31u) == 0u) emit_speciation(l, k);
+    return result;
+}
+
+// A lineage's round by one warp: chain_run where it applies, else coop_run.
+template <int KIND>
+__device__ __forceinline__ int warp_run(Lane &l, const SimParams &p, const EventSink &k, uint64_t &events,
+                                        const volatile unsigned *stop = nullptr) {
+    if constexpr (kChainKind<KIND>) {
+        if (chain_takes<KIND>(p, l)) return chain_run<KIND>(l, p, k, events, stop);
+    }
+    return coop_run<KIND>(l, p, k, events, stop);
+}
+
 __device__ __forceinline__ EventSink sink_of(const StepArgs &a) {
     EventSink k;
     k.spec = a.spec;
@@ -1046,7 +1423,7 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
                 }
                 if (r == kStepSpeciated) warp_steps += 1;
             } else {
-                r = coop_run<KIND>(c, p, sink, warp_steps);
+                r = warp_run<KIND>(c, p, sink, warp_steps);
             }
             // the lineage's own round is done: it no longer holds the launch
             if (a.busy && lane_id == 0) atomicSub(a.busy, 1u);
@@ -1072,7 +1449,7 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
                     __syncwarp();
                     c.horizon = h;
                     // interrupted at a peek once the launch's regular work is done
-                    r = coop_run<KIND>(c, p, sink, warp_steps, SINGLE ? nullptr : a.busy);
+                    r = warp_run<KIND>(c, p, sink, warp_steps, SINGLE ? nullptr : a.busy);
                     if (r == kStepStop && __double_as_longlong(c.next) < __double_as_longlong(h)) {
                         // the round is not finished: give it back, so the
                         // scheduler sets (and counts) the same horizon again
@@ -1329,7 +1706,7 @@ __global__ void __launch_bounds__(THREADS, 1) resident_kernel(ResidentArgs a) {
                         }
                     } else {
                         uint64_t ev = 0;
-                        c_live = coop_run<KIND>(c, p, sink, ev) == kStepStop;
+                        c_live = warp_run<KIND>(c, p, sink, ev) == kStepStop;
                         my_events += ev;
                     }
                     if ((t & 31u) == 0) {

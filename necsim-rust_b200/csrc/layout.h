@@ -134,7 +134,7 @@ struct alignas(16) SimParams {
     uint64_t step_slice_max;
     uint64_t lineage_offset;  // first slot of the simulation's resident-arena segment
     int32_t resident;         // 1 once the resident kernel owns the simulation
-    int32_t pad1;
+    int32_t chain;            // 1: chain_run may step the simulation's lineages (kernels.cu)
     int32_t active;           // 1 while the simulation still advances
     int32_t pad;
 };

@@ -1,0 +1,108 @@
+"""The lone-lineage kernel form (chain_run) at the edges of its rule: worlds of
+one cell, 2^32 - 1 cells and beyond, a metacommunity that reaches into the
+local extent, time buckets with many events or almost none, delta_t that is no
+power of two (the general form), every event a speciation or a migration,
+interrupted rounds and wide displacements, all against the oracle's canonical
+schedule bit for bit."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import same_stream
+
+pytestmark = pytest.mark.gpu
+
+M32 = 0xFFFFFFFF
+
+
+def ns(w, h, deme, nu):
+    return dict(kind=0, speciation_probability=nu, width=w, height=h, deme=deme)
+
+
+def si(local, deme, meta, meta_deme, migration, nu, height=1, meta_height=1):
+    return dict(kind=1, speciation_probability=nu, width=local, height=height, deme=deme, meta_width=meta,
+                meta_height=meta_height, meta_deme=meta_deme, migration_probability=migration)
+
+
+def ai(radius, sigma, nu, centre=(M32 // 2, M32 // 2)):
+    return dict(kind=2, speciation_probability=nu, sigma=sigma, radius=radius, centre_x=centre[0],
+                centre_y=centre[1])
+
+
+CASES = {
+    # name: (scenario, kernel arguments, resumed lineages (None: every origin))
+    "one_cell": (ns(1, 1, 1, 0.02), {}, None),
+    "one_column": (ns(1, 37, 3, 0.01), {}, None),
+    "every_event_speciates": (ns(9, 5, 2, 1.0), {}, None),
+    "cells_below_2_32": (ns(65535, 65537, 7, 0.01), {}, 40),   # 2^32 - 1 cells
+    "cells_2_32": (ns(65536, 65536, 7, 0.01), {}, 40),         # the general form
+    "cells_above_2_32": (ns(M32, 3, 2, 0.01), {}, 40),
+    "many_events_per_bucket": (ns(20, 11, 3, 0.004), dict(delta_t=32.0), None),
+    "four_events_per_bucket": (ns(20, 11, 3, 0.004), dict(delta_t=8.0), None),
+    "few_events_per_bucket": (ns(12, 7, 3, 0.01), dict(delta_t=0.0625), None),
+    "delta_t_no_power_of_two": (ns(20, 11, 3, 0.004), dict(delta_t=3.0), None),
+    "short_rounds": (ns(20, 11, 3, 0.004), dict(step_slice=1, min_round_events=1), None),
+    "local_only_by_chance": (si(15, 2, 1000, 3, 1e-3, 0.01), {}, None),
+    "every_event_migrates": (si(15, 2, 1000, 3, 1.0, 0.01), {}, None),
+    "demes_and_rows": (si(6, 5, 40, 4, 0.2, 0.01, height=4, meta_height=9), {}, None),
+    "meta_inside_local": (si(50, 2, M32, 3, 0.3, 0.01), {}, None),
+    "meta_cells_above_2_32": (si(50, 2, 70000, 3, 0.3, 0.01, meta_height=70000), {}, None),
+    "meta_many_events": (si(15, 2, 1000, 3, 0.1, 0.01), dict(delta_t=16.0), None),
+    "wide_displacements": (ai(4, 3e8, 0.01), {}, None),
+    "no_displacement": (ai(4, 0.0, 0.01, centre=(1, M32)), {}, None),
+    "narrow_displacements": (ai(5, 0.4, 0.01, centre=(1, M32)), {}, None),
+    "clark_wide": (dict(kind=4, speciation_probability=0.01, shape_u=1e9, tail_p=1.0, radius=4, centre_x=2,
+                        centre_y=M32 - 1), {}, None),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+@pytest.mark.parametrize("batch", [False, True])
+def test_matches_oracle(nb, syn, oracle, name, batch):
+    desc, kw, resumed = CASES[name]
+    oracle_kw = dict(dict(step_slice=10, min_round_events=1 << 20), **kw)
+    if resumed is not None:
+        lins = np.zeros(resumed, dtype=nb.LINEAGE_DTYPE)
+        u = syn.splitmix64(3, 3 * resumed)
+        lins["x"] = u[:resumed] % np.uint64(desc["width"])
+        lins["y"] = u[resumed:2 * resumed] % np.uint64(desc["height"])
+        lins["index"] = u[2 * resumed:] % np.uint64(desc["deme"])
+        lins["gref"] = np.arange(resumed)
+        if batch:
+            pytest.skip("batches start from every origin")
+        with nb.Simulation(syn.to_scenario(desc), desc["speciation_probability"], nb.CUDA(**kw)) as sim:
+            g = sim.resume(lins, 0.0, 5)
+        c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, lineages=lins, step_slice_max=1024, **oracle_kw)
+    elif batch:
+        # beside another simulation and in the resident kernel
+        other = dict(desc, speciation_probability=min(1.0, 2.0 * desc["speciation_probability"]))
+        pair = [desc, other]
+        g = nb.simulate_batch([syn.to_scenario(d) for d in pair], [d["speciation_probability"] for d in pair],
+                              [5, 6], nb.CUDA(resident=True, **kw), collect=True)[0]
+        c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice_max=1024, **oracle_kw)
+    else:
+        with nb.Simulation(syn.to_scenario(desc), desc["speciation_probability"], nb.CUDA(**kw)) as sim:
+            g = sim.simulate(5)
+        c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice_max=1024, **oracle_kw)
+    assert same_stream(g.speciation, c.speciation)
+    assert (g.steps, g.n_rounds, g.n_dedup, g.time) == (c.steps, c.n_rounds, c.n_dedup, c.time)
+
+
+@pytest.mark.parametrize("name", ["four_events_per_bucket", "demes_and_rows", "narrow_displacements"])
+@pytest.mark.parametrize("pause", [7.25, 40.0])
+def test_pause_and_dispersal_events(nb, syn, oracle, name, pause):
+    """The peek kept over a pause, and every executed event reported."""
+    desc, kw, _ = CASES[name]
+    algo = nb.CUDA(report_dispersal=True, **kw)
+    with nb.Simulation(syn.to_scenario(desc), desc["speciation_probability"], algo) as sim:
+        g = sim.simulate(5, pause_before=pause)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice=10, min_round_events=1 << 20,
+                        step_slice_max=1024, pause_before=pause, report_dispersal=True, dispersal_cap=1 << 20, **kw)
+    assert same_stream(g.speciation, c.speciation)
+    a = np.sort(g.dispersal, order=("event_time", "gref"))
+    b = np.sort(c.dispersal, order=("event_time", "gref"))
+    assert len(a) == len(b) > 0
+    for f in ("gref", "prior_time", "event_time", "x", "y", "index", "tx", "ty", "tindex"):
+        assert np.array_equal(a[f], b[f]), f
+    rem, crem = np.sort(g.remaining, order="gref"), np.sort(c.remaining, order="gref")
+    for f in ("gref", "x", "y", "index", "last_event_time"):
+        assert np.array_equal(rem[f], crem[f]), f
