@@ -347,6 +347,7 @@ struct SimHost {
     uint64_t lineage_offset;  // first slot in the batch's lineage arrays
     double start_time;        // min last event time of its lineages
     double start_max;         // max last event time of its lineages
+    const necsim_lineage *noise_origins;  // WrappingNoise: its origins on the device (owned by the engine)
     SimParams params;
 };
 
@@ -424,6 +425,26 @@ void validate(const necsim_scenario &sc) {
     }
 }
 
+// floor(sqrt(v)), v < 2^33
+uint64_t isqrt(uint64_t v) {
+    uint64_t r = (uint64_t)std::sqrt((double)v);
+    while (r * r > v) --r;
+    while ((r + 1) * (r + 1) <= v) ++r;
+    return r;
+}
+
+// Lengths of the rows of an AlmostInfinite Circle sample
+// (origin_sampler/singleton_demes/circle.rs:36-70, 100-140) as prefix sums:
+// dx^2 + dy^2 <= r^2 row by row.
+std::vector<uint64_t> circle_rows(uint32_t radius) {
+    const int64_t r = radius;
+    std::vector<uint64_t> prefix;
+    prefix.reserve((size_t)(2 * r + 2));
+    prefix.push_back(0);
+    for (int64_t dy = -r; dy <= r; ++dy) prefix.push_back(prefix.back() + 2 * isqrt((uint64_t)(r * r - dy * dy)) + 1);
+    return prefix;
+}
+
 // Number of origin lineages of the scenario (OriginPreSampler::all()).
 uint64_t count_origins(const necsim_scenario &sc) {
     switch (sc.kind) {
@@ -433,12 +454,7 @@ uint64_t count_origins(const necsim_scenario &sc) {
     case NECSIM_ALMOST_INFINITE_NORMAL:
     case NECSIM_ALMOST_INFINITE_CLARK2DT: {
         if (sc.sample_width) return sc.sample_width * sc.sample_height;  // Rectangle: every location
-        const int64_t r = sc.radius;
-        uint64_t n = 0;
-        for (int64_t dy = -r; dy <= r; ++dy)
-            for (int64_t dx = -r; dx <= r; ++dx)
-                if ((uint64_t)(dx * dx + dy * dy) <= (uint64_t)(r * r)) ++n;
-        return n;
+        return circle_rows(sc.radius).back();
     }
     case NECSIM_WRAPPING_NOISE: {
         uint64_t n = 0;
@@ -452,6 +468,13 @@ uint64_t count_origins(const necsim_scenario &sc) {
         return n;
     }
     }
+}
+
+// The origin count a simulation is set up with: WrappingNoise origins are
+// found and counted on the device (prepare_engine) unless the learned
+// schedule scores the simulations by it first.
+uint64_t setup_origins(const necsim_scenario &sc, const necsim_args &args) {
+    return sc.kind == NECSIM_WRAPPING_NOISE && args.schedule == 0 ? 0 : count_origins(sc);
 }
 
 // ceil(2^64 / d) for 1 < d < 2^32, 0 for d <= 1 (quotient = dividend)
@@ -580,30 +603,36 @@ necsim_args with_defaults(const necsim_args *in) {
 }
 
 // ---- device buffers of one (batched) simulation ----
+
+// Hands out 256-byte aligned pieces of one allocation, or only adds up their
+// size (base null).
+struct Carver {
+    unsigned char *base = nullptr;
+    size_t bytes = 0;
+    template <typename T>
+    T *take(size_t n) {
+        T *p = base ? reinterpret_cast<T *>(base + bytes) : nullptr;
+        bytes += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
+        return p;
+    }
+};
+
 struct DeviceLineages {
     LineageSoA soa{};
     uint8_t *state = nullptr;
-    void alloc(uint64_t n, bool with_pred = false) {
-        if (with_pred) soa.pred_end = dev_alloc<float>(n);
-        soa.x = dev_alloc<uint32_t>(n);
-        soa.y = dev_alloc<uint32_t>(n);
-        soa.idx = dev_alloc<uint32_t>(n);
-        soa.sim = dev_alloc<uint32_t>(n);
-        soa.last = dev_alloc<double>(n);
-        soa.next = dev_alloc<double>(n);
-        soa.reprime = dev_alloc<uint64_t>(n);
-        soa.gref = dev_alloc<uint64_t>(n);
-        soa.steps = dev_alloc<uint64_t>(n);
-        soa.has_next = dev_alloc<uint8_t>(n);
-        state = dev_alloc<uint8_t>(n);
-    }
-    void release() {
-        void *ptrs[] = {soa.x, soa.y, soa.idx, soa.sim, soa.last, soa.next, soa.reprime,
-                        soa.gref, soa.steps, soa.has_next, state, soa.pred_end};
-        for (void *p : ptrs)
-            if (p) cudaFree(p);
-        soa = LineageSoA{};
-        state = nullptr;
+    void carve(Carver &c, uint64_t n, bool with_pred = false) {
+        soa.pred_end = with_pred ? c.take<float>(n) : nullptr;
+        soa.x = c.take<uint32_t>(n);
+        soa.y = c.take<uint32_t>(n);
+        soa.idx = c.take<uint32_t>(n);
+        soa.sim = c.take<uint32_t>(n);
+        soa.last = c.take<double>(n);
+        soa.next = c.take<double>(n);
+        soa.reprime = c.take<uint64_t>(n);
+        soa.gref = c.take<uint64_t>(n);
+        soa.steps = c.take<uint64_t>(n);
+        soa.has_next = c.take<uint8_t>(n);
+        state = c.take<uint8_t>(n);
     }
 };
 
@@ -646,9 +675,17 @@ struct Engine {
     std::vector<CellRecord *> d_cells;
     std::vector<AliasAtom *> d_atoms;
 
+    // the run's buffers, carved from one allocation for n_cap lineages
+    unsigned char *arena = nullptr;
+    size_t arena_bytes = 0;
+    uint64_t n_cap = 0;
     DeviceLineages A, B;
     DeviceLineages R;  // resident arena: small simulations' lineages, one segment each
-    LineageSoA O{};  // resident origins (x, y, idx, sim, last, gref)
+    // how every simulation's origins are written (origins.cu), and the prefix
+    // sums and lineages that the descriptions point to
+    OriginSpec *d_specs = nullptr;
+    std::vector<uint64_t *> d_prefix;
+    std::vector<necsim_lineage *> d_given;
     cudaEvent_t ev_res0 = nullptr, ev_res1 = nullptr;
     uint64_t h2d_bytes = 0, d2h_bytes = 0;  // host<->device traffic of the current call
     uint32_t *owner = nullptr, *slot = nullptr;
@@ -705,6 +742,14 @@ struct Engine {
 
     ~Engine() { release(); }
 
+    // Frees what a run's origins were described with.
+    void drop_inputs() {
+        for (auto p : d_prefix) cudaFree(p);
+        for (auto p : d_given) cudaFree(p);
+        d_prefix.clear();
+        d_given.clear();
+    }
+
     void release() {
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         graph_exec = nullptr;
@@ -715,26 +760,13 @@ struct Engine {
         if (ev_total0) cudaEventDestroy(ev_total0);
         if (ev_total1) cudaEventDestroy(ev_total1);
         ev_total0 = ev_total1 = nullptr;
-        A.release();
-        B.release();
-        R.release();
         if (ev_res0) cudaEventDestroy(ev_res0);
         if (ev_res1) cudaEventDestroy(ev_res1);
         ev_res0 = ev_res1 = nullptr;
-        void *optrs[] = {O.x, O.y, O.idx, O.sim, O.last, O.gref};
-        for (void *p : optrs)
-            if (p) cudaFree(p);
-        O = LineageSoA{};
-        void *ptrs[] = {owner, slot, min_gref, d_params, d_counters, d_ctl, d_spec, d_disp};
-        for (void *p : ptrs)
-            if (p) cudaFree(p);
-        owner = slot = nullptr;
-        min_gref = nullptr;
-        d_params = nullptr;
-        d_counters = nullptr;
-        d_ctl = nullptr;
-        d_spec = nullptr;
-        d_disp = nullptr;
+        if (arena) cudaFree(arena);
+        arena = nullptr;
+        arena_bytes = 0;
+        drop_inputs();
         for (auto p : d_cells)
             if (p) cudaFree(p);
         for (auto p : d_atoms)
@@ -747,12 +779,9 @@ struct Engine {
         d_atoms.clear();
         d_entropy.clear();
         d_turnover.clear();
-        void *lptrs[] = {order_keys, order_hist, order, trace_rows, trace_deaths, trace_counts};
+        void *lptrs[] = {trace_rows, trace_deaths, trace_counts};
         for (void *p : lptrs)
             if (p) cudaFree(p);
-        order_keys = nullptr;
-        order_hist = nullptr;
-        order = nullptr;
         trace_rows = nullptr;
         trace_deaths = nullptr;
         trace_counts = nullptr;
@@ -834,6 +863,8 @@ void setup_engine(Engine &E, const necsim_args &args, int stream_priority = 0) {
     CK(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreate(&E.ev_total0));
     CK(cudaEventCreate(&E.ev_total1));
+    CK(cudaEventCreate(&E.ev_res0));
+    CK(cudaEventCreate(&E.ev_res1));
     void *h = nullptr;
     CK(cudaMallocHost(&h, sizeof(Control)));
     E.h_ctl = static_cast<Control *>(h);
@@ -860,46 +891,59 @@ void choose_launch(Engine &E) {
     E.aux_grid = (unsigned)(E.n_sms * 8);
 }
 
-void alloc_run_buffers(Engine &E) {
-    const uint64_t n = E.n_total;
-    E.A.alloc(n, E.learned);
-    E.R.alloc(n);
-    CK(cudaEventCreate(&E.ev_res0));
-    CK(cudaEventCreate(&E.ev_res1));
-    E.B.alloc(n, E.learned);
+void carve_run_buffers(Engine &E, Carver &c) {
+    const uint64_t n = E.n_cap;
+    E.A.carve(c, n, E.learned);
+    E.B.carve(c, n, E.learned);
+    if (E.args.resident) E.R.carve(c, n);
     if (E.learned) {
-        E.order_keys = dev_alloc<uint8_t>(n);
-        E.order = dev_alloc<uint32_t>(n);
-        E.order_hist = dev_alloc<unsigned>(2 * kOrderBuckets);
-        CK(cudaMemsetAsync(E.order_hist, 0, 2 * kOrderBuckets * sizeof(unsigned), E.stream));
+        E.order_keys = c.take<uint8_t>(n);
+        E.order = c.take<uint32_t>(n);
+        E.order_hist = c.take<unsigned>(2 * kOrderBuckets);
     }
-    if (E.tracing) {
-        E.trace_deaths_cap = n;
-        E.trace_deaths = dev_alloc<TraceDeath>(n);
-        E.trace_rows = dev_alloc<TraceRow>(E.trace_rows_cap);
-        E.trace_counts = dev_alloc<unsigned long long>(2);
-        CK(cudaMemsetAsync(E.trace_counts, 0, 2 * sizeof(unsigned long long), E.stream));
-    }
-    unsigned long long want = (n * E.args.dedup_factor_pct + 99) / 100;
+    E.owner = c.take<uint32_t>(E.table_size);
+    E.min_gref = c.take<unsigned long long>(E.table_size);
+    E.slot = c.take<uint32_t>(n);
+    E.d_params = c.take<SimParams>(E.sims.size());
+    E.d_specs = c.take<OriginSpec>(E.sims.size());
+    E.d_counters = c.take<SimCounters>(E.sims.size());
+    E.d_ctl = c.take<Control>(1);
+    E.d_spec = c.take<DevSpeciationEvent>(n);
+    E.d_disp = E.disp_cap ? c.take<DevDispersalEvent>(E.disp_cap) : nullptr;
+}
+
+// The run's buffers for n_cap lineages (at least n_total), as one allocation:
+// some forty separate ones and their frees took longer than a small run.
+void alloc_run_buffers(Engine &E, uint64_t n_cap) {
+    E.n_cap = n_cap;
+    E.spec_cap = n_cap;
+    unsigned long long want = (n_cap * E.args.dedup_factor_pct + 99) / 100;
     if (want < 2) want = 2;
     unsigned long long size = 1;
     while (size < want) size <<= 1;
     E.table_size = size;
-    E.owner = dev_alloc<uint32_t>(size);
-    E.min_gref = dev_alloc<unsigned long long>(size);
-    E.slot = dev_alloc<uint32_t>(n);
+    Carver c;
+    carve_run_buffers(E, c);
+    E.arena = dev_alloc<unsigned char>(c.bytes);
+    E.arena_bytes = c.bytes;
+    c = Carver{};
+    c.base = E.arena;
+    carve_run_buffers(E, c);
+    if (E.tracing) {
+        E.trace_deaths_cap = n_cap;
+        E.trace_deaths = dev_alloc<TraceDeath>(n_cap);
+        E.trace_rows = dev_alloc<TraceRow>(E.trace_rows_cap);
+        E.trace_counts = dev_alloc<unsigned long long>(2);
+        CK(cudaMemsetAsync(E.trace_counts, 0, 2 * sizeof(unsigned long long), E.stream));
+    }
+    if (E.learned) CK(cudaMemsetAsync(E.order_hist, 0, 2 * kOrderBuckets * sizeof(unsigned), E.stream));
+    // every round leaves the table empty
     CK(cudaMemsetAsync(E.owner, 0xff, size * sizeof(uint32_t), E.stream));
     CK(cudaMemsetAsync(E.min_gref, 0xff, size * sizeof(unsigned long long), E.stream));
-    E.d_params = dev_alloc<SimParams>(E.sims.size());
-    E.d_counters = dev_alloc<SimCounters>(E.sims.size());
-    E.d_ctl = dev_alloc<Control>(1);
     // each run resets both; a run without lineages runs no round and reads
     // them as they are here (upload_origins synchronises the stream next)
     CK(cudaMemsetAsync(E.d_counters, 0, E.sims.size() * sizeof(SimCounters), E.stream));
     CK(cudaMemsetAsync(E.d_ctl, 0, sizeof(Control), E.stream));
-    E.spec_cap = n;
-    E.d_spec = dev_alloc<DevSpeciationEvent>(n);
-    if (E.disp_cap) E.d_disp = dev_alloc<DevDispersalEvent>(E.disp_cap);
 }
 
 // Calls push(x, y, index, global_reference) for every origin lineage of the
@@ -1013,75 +1057,107 @@ std::vector<float> score_simulations(necsim_model *m, const std::vector<SimHost>
     return score;
 }
 
-// Builds the origin lineages of every simulation on the host, in the
-// reference's origin-sampler order, and uploads them as structure of arrays.
-void upload_origins(Engine &E, const std::vector<std::vector<necsim_lineage>> *given) {
-    const uint64_t n = E.n_total;
-    std::vector<uint32_t> x(n), y(n), idx(n), sim(n);
-    std::vector<double> last(n);
-    std::vector<uint64_t> gref(n);
-    for (size_t s = 0; s < E.sims.size(); ++s) {
-        SimHost &sh = E.sims[s];
-        uint64_t o = sh.lineage_offset;
-        double tmin = 0.0, tmax = 0.0;
-        bool first = true;
-        auto push = [&](uint32_t xx, uint32_t yy, uint32_t ii, uint64_t g, double t) {
-            x[o] = xx;
-            y[o] = yy;
-            idx[o] = ii;
-            sim[o] = (uint32_t)s;
-            last[o] = t;
-            gref[o] = g;
-            ++o;
-            if (first || t < tmin) tmin = t;
-            if (first || t > tmax) tmax = t;
-            first = false;
-        };
-        const necsim_scenario &sc = sh.sc;
-        if (given) {
-            for (const necsim_lineage &l : (*given)[s]) push(l.x, l.y, l.index, l.global_reference, l.last_event_time);
-        } else {
-            for_each_origin(sc, [&](uint32_t xx, uint32_t yy, uint32_t ii, uint64_t g) { push(xx, yy, ii, g, 0.0); });
+// The WrappingNoise origins of a simulation, found on the device (E.d_given
+// owns the list): its n_origins and the lineages.
+const necsim_lineage *find_noise_origins(Engine &E, SimHost &sh) {
+    const necsim_scenario &sc = sh.sc;
+    const uint64_t n = sc.sample_width * sc.sample_height;
+    struct Scratch {
+        NoiseHabitat *h = nullptr;
+        unsigned long long *count = nullptr;
+        ~Scratch() {
+            if (h) cudaFree(h);
+            if (count) cudaFree(count);
         }
-        if (o != sh.lineage_offset + sh.n_origins) fail(NECSIM_E_INVALID_ARGUMENT, "origin count mismatch");
-        sh.start_time = tmin;
-        sh.start_max = tmax;
-    }
-    // resident copy of the origins: every run starts from it
-    LineageSoA &d = E.O;
-    d.x = dev_alloc<uint32_t>(n);
-    d.y = dev_alloc<uint32_t>(n);
-    d.idx = dev_alloc<uint32_t>(n);
-    d.sim = dev_alloc<uint32_t>(n);
-    d.last = dev_alloc<double>(n);
-    d.gref = dev_alloc<uint64_t>(n);
-    CK(cudaMemcpyAsync(d.x, x.data(), n * 4, cudaMemcpyHostToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.y, y.data(), n * 4, cudaMemcpyHostToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.idx, idx.data(), n * 4, cudaMemcpyHostToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.sim, sim.data(), n * 4, cudaMemcpyHostToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.last, last.data(), n * 8, cudaMemcpyHostToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.gref, gref.data(), n * 8, cudaMemcpyHostToDevice, E.stream));
-    E.h2d_bytes += n * (4 * 4 + 8 * 2);
-    CK(cudaStreamSynchronize(E.stream));
+    } d;
+    d.h = dev_alloc<NoiseHabitat>(1);
+    d.count = dev_alloc<unsigned long long>(1);
+    CK(cudaMemcpyAsync(d.h, &sh.params.noise, sizeof(NoiseHabitat), cudaMemcpyHostToDevice, E.stream));
+    auto pass = [&](necsim_lineage *out) {
+        unsigned long long found = 0;
+        CK(cudaMemsetAsync(d.count, 0, sizeof(found), E.stream));
+        CK(launch_noise_origins(d.h, sc.sample_x, sc.sample_y, sc.sample_width, n, out, d.count,
+                                (unsigned)E.n_sms * 16u, E.stream));
+        CK(cudaMemcpyAsync(&found, d.count, sizeof(found), cudaMemcpyDeviceToHost, E.stream));
+        CK(cudaStreamSynchronize(E.stream));
+        return (uint64_t)found;
+    };
+    sh.n_origins = pass(nullptr);
+    if (sh.n_origins >= 0xffffffffULL) fail(NECSIM_E_TOO_LARGE, "more than 2^32 - 1 lineages");
+    necsim_lineage *out = dev_alloc<necsim_lineage>(sh.n_origins);
+    E.d_given.push_back(out);
+    if (pass(out) != sh.n_origins) fail(NECSIM_E_DEVICE_CHECK, "origin count mismatch");
+    E.h2d_bytes += sizeof(NoiseHabitat);
+    return out;
 }
 
-// Resets the working lineages to the resident origins (device to device).
+// Describes every simulation's origin lineages to the device (origins.cu
+// writes them at the start of each run) and uploads what the description
+// needs: row or cell prefix sums, or the caller's lineages.
+void upload_origins(Engine &E, const std::vector<std::vector<necsim_lineage>> *given) {
+    std::vector<OriginSpec> specs(E.sims.size());
+    auto upload = [&](auto &list, const auto &v) {
+        using T = typename std::decay_t<decltype(v)>::value_type;
+        T *d = dev_alloc<T>(v.size());
+        list.push_back(d);
+        if (!v.empty()) CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, E.stream));
+        CK(cudaStreamSynchronize(E.stream));  // v may go
+        E.h2d_bytes += v.size() * sizeof(T);
+        return d;
+    };
+    for (size_t s = 0; s < E.sims.size(); ++s) {
+        SimHost &sh = E.sims[s];
+        const necsim_scenario &sc = sh.sc;
+        OriginSpec &o = specs[s];
+        std::memset(&o, 0, sizeof(o));
+        o.offset = sh.lineage_offset;
+        o.n = sh.n_origins;
+        o.width = sc.width;
+        o.deme = sc.deme;
+        sh.start_time = sh.start_max = 0.0;
+        if (given) {
+            const std::vector<necsim_lineage> &v = (*given)[s];
+            o.form = kOriginGiven;
+            o.given = upload(E.d_given, v);
+            for (size_t j = 0; j < v.size(); ++j) {
+                sh.start_time = j ? std::min(sh.start_time, v[j].last_event_time) : v[j].last_event_time;
+                sh.start_max = j ? std::max(sh.start_max, v[j].last_event_time) : v[j].last_event_time;
+            }
+        } else if (sc.kind == NECSIM_NON_SPATIAL || sc.kind == NECSIM_SPATIALLY_IMPLICIT) {
+            o.form = kOriginGrid;
+        } else if (sc.kind == NECSIM_WRAPPING_NOISE) {
+            o.form = kOriginGiven;
+            o.given = sh.noise_origins;
+        } else if (sc.kind == NECSIM_SPATIALLY_EXPLICIT) {
+            o.form = kOriginCells;
+            const uint64_t cells = (uint64_t)sc.width * sc.height;
+            std::vector<uint64_t> prefix(cells + 1, 0);
+            for (uint64_t c = 0; c < cells; ++c) prefix[c + 1] = prefix[c] + sc.habitat[c];
+            o.rows = cells;
+            o.prefix = upload(E.d_prefix, prefix);
+        } else if (sc.sample_width) {
+            o.form = kOriginPlane;
+            o.width = sc.sample_width;
+            o.x0 = sc.sample_x;
+            o.y0 = sc.sample_y;
+        } else {
+            o.form = kOriginCircle;
+            const std::vector<uint64_t> prefix = circle_rows(sc.radius);
+            o.rows = prefix.size() - 1;
+            o.x0 = sc.centre_x;
+            o.y0 = sc.centre_y - sc.radius;
+            o.prefix = upload(E.d_prefix, prefix);
+        }
+    }
+    CK(cudaMemcpyAsync(E.d_specs, specs.data(), specs.size() * sizeof(OriginSpec), cudaMemcpyHostToDevice, E.stream));
+    CK(cudaStreamSynchronize(E.stream));
+    E.h2d_bytes += specs.size() * sizeof(OriginSpec);
+}
+
+// The working lineages at the start of a run: every simulation's origins.
 void reset_lineages(Engine &E) {
-    const uint64_t n = E.n_total;
-    LineageSoA &d = E.A.soa;
-    const LineageSoA &o = E.O;
-    CK(cudaMemcpyAsync(d.x, o.x, n * 4, cudaMemcpyDeviceToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.y, o.y, n * 4, cudaMemcpyDeviceToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.idx, o.idx, n * 4, cudaMemcpyDeviceToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.sim, o.sim, n * 4, cudaMemcpyDeviceToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.last, o.last, n * 8, cudaMemcpyDeviceToDevice, E.stream));
-    CK(cudaMemcpyAsync(d.gref, o.gref, n * 8, cudaMemcpyDeviceToDevice, E.stream));
-    CK(cudaMemsetAsync(d.steps, 0, n * 8, E.stream));
-    CK(cudaMemsetAsync(d.has_next, 0, n, E.stream));
-    CK(cudaMemsetAsync(d.next, 0, n * 8, E.stream));
-    CK(cudaMemsetAsync(d.reprime, 0, n * 8, E.stream));
-    CK(cudaMemsetAsync(E.A.state, 0, n, E.stream));
-    if (d.pred_end) CK(cudaMemsetAsync(d.pred_end, 0, n * sizeof(float), E.stream));
+    CK(launch_origins(E.d_specs, (uint32_t)E.sims.size(), E.n_total, E.A.soa, E.A.state, (unsigned)E.n_sms * 8u,
+                      E.stream));
 }
 
 StepArgs make_step_args(Engine &E, DeviceLineages &in) {
@@ -1826,6 +1902,8 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
         if (args.model->device != E.device) fail(NECSIM_E_INVALID_ARGUMENT, "the model lives on another device");
         E.model_w = args.model->w;
     }
+    if (E.kind == NECSIM_WRAPPING_NOISE && !given)
+        for (auto &sh : sims) sh.noise_origins = find_noise_origins(E, sh);
     if (args.report_dispersal) {
         // every lineage stays in the global rounds, which drain the events
         // after each round; the buffer holds twice a round's expected events
@@ -1872,7 +1950,7 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
     // gives a simulation one SM)
     if (E.sims.size() == 1) E.args.resident = 0;
     choose_launch(E);
-    alloc_run_buffers(E);
+    alloc_run_buffers(E, E.n_total);
     upload_origins(E, given);
     if (E.n_total > 0) build_graph(E);
 }
@@ -2266,7 +2344,7 @@ static int simulate_impl(necsim_ctx *ctx, const necsim_lineage *lineages, uint64
             sh.n_origins = keep.size();
             given.push_back(std::move(keep));
         } else {
-            sh.n_origins = count_origins(ctx->scenario);
+            sh.n_origins = setup_origins(ctx->scenario, ctx->args);
         }
         std::vector<SimHost> sims{sh};
         necsim_outcome o;
@@ -2314,7 +2392,7 @@ int necsim_gpu_simulate_batch(const necsim_scenario *scenarios, const uint64_t *
             sh.seed = wyhash_seeds[s];
             sh.params = base_params(scenarios[s], args, wyhash_seeds[s]);
             sh.params.pause_before = pause_before >= 0.0 ? pause_before : -1.0;
-            sh.n_origins = count_origins(scenarios[s]);
+            sh.n_origins = setup_origins(scenarios[s], args);
         }
         BatchRun b;
         prepare_batch(b, std::move(sims), args);
@@ -2349,7 +2427,7 @@ static std::vector<SimHost> batch_sims(const necsim_scenario *scenarios, const u
         sh.seed = wyhash_seeds[s];
         sh.params = base_params(scenarios[s], args, wyhash_seeds[s]);
         sh.params.pause_before = pause_before >= 0.0 ? pause_before : -1.0;
-        sh.n_origins = count_origins(scenarios[s]);
+        sh.n_origins = setup_origins(scenarios[s], args);
     }
     return sims;
 }

@@ -8,6 +8,8 @@
 #include "layout.h"
 #include "learned.h"
 
+struct necsim_lineage;
+
 namespace necsim {
 
 constexpr int kStepBlockMax = 256;
@@ -135,6 +137,30 @@ struct ResidentArgs {
 // The SM ids present on the device: bit smid of mask[smid / 32] is set by a
 // block that ran there (grid blocks of 32 threads; mask zeroed before).
 cudaError_t launch_sm_census(uint32_t *mask, unsigned grid, cudaStream_t st);
+
+// The origin lineages of one simulation (origins.cu), written to slots
+// offset .. offset + n of the round's structure of arrays.
+enum : int32_t {
+    kOriginGrid = 0,    // width x ..., `deme` individuals per cell, position order (NonSpatial, SpatiallyImplicit)
+    kOriginPlane = 1,   // an AlmostInfinite rectangle at (x0, y0), wrapping at 2^32
+    kOriginCircle = 2,  // an AlmostInfinite circle: rows from y0, centred on x0, prefix sums of their lengths
+    kOriginCells = 3,   // SpatiallyExplicit: prefix sums of the habitat over the cells
+    kOriginGiven = 4,   // lineages handed over by the caller (or found by noise_origins)
+};
+struct OriginSpec {
+    int32_t form;
+    uint32_t deme, x0, y0;
+    uint64_t offset, n, width, rows;
+    const uint64_t *prefix;               // rows + 1 entries
+    const struct ::necsim_lineage *given;
+};
+cudaError_t launch_origins(const OriginSpec *specs, uint32_t n_sims, uint64_t n_total, const LineageSoA &out,
+                           uint8_t *state, unsigned grid, cudaStream_t st);
+// the habitable locations among n of a WrappingNoise sample: counted in
+// *count (zero before) and, when out is not null, written there in any order
+cudaError_t launch_noise_origins(const NoiseHabitat *habitat, uint32_t x0, uint32_t y0, uint64_t width, uint64_t n,
+                                 struct ::necsim_lineage *out, unsigned long long *count, unsigned grid,
+                                 cudaStream_t st);
 
 cudaError_t launch_resident(int kind, const ResidentArgs &a, unsigned grid, cudaStream_t st);
 cudaError_t launch_promote(SimParams *params, uint32_t n_sims, cudaStream_t st);
