@@ -254,6 +254,9 @@ int necsim_gpu_create(const necsim_scenario *scenario, const necsim_args *args,
  * until `pause_before` (< 0: no pause).  `wyhash_seed` is the WyHash seed
  * word (necsim/impls/no-std/src/cogs/rng/wyhash.rs:41-49); use
  * necsim_seed_from_u64() for the reference's `rng: Seed(u64)`.
+ * The device workspace of a finished call (at most 1/32 of the device's
+ * memory, four calls' worth) is kept for later calls on any context; it is
+ * freed when a device allocation of the library fails.
  * Replaces `Algorithm::initialise_and_simulate` (algorithms/src/lib.rs:81-93). */
 int necsim_gpu_simulate(necsim_ctx *ctx, uint64_t wyhash_seed, double pause_before,
                         const necsim_reporter *reporter, necsim_outcome *outcome);

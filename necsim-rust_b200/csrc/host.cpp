@@ -66,10 +66,17 @@ struct ApiError {
 
 [[noreturn]] void fail(int code, const std::string &msg) { throw ApiError{code, msg}; }
 
+// Frees the workspaces kept between calls (EnginePool below).
+bool release_idle_workspaces();
+
 template <typename T>
 T *dev_alloc(size_t n) {
     void *p = nullptr;
     cudaError_t e = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T));
+    if (e == cudaErrorMemoryAllocation && release_idle_workspaces()) {
+        cudaGetLastError();
+        e = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T));
+    }
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         fail(NECSIM_E_OUT_OF_MEMORY, "device allocation of " + std::to_string(n * sizeof(T)) + " bytes failed");
@@ -679,6 +686,8 @@ struct Engine {
     unsigned char *arena = nullptr;
     size_t arena_bytes = 0;
     uint64_t n_cap = 0;
+    uint64_t disp_room = 0;             // dispersal events that d_disp holds
+    unsigned long long context = 0;     // CUDA context id while idle in the EnginePool
     DeviceLineages A, B;
     DeviceLineages R;  // resident arena: small simulations' lineages, one segment each
     // how every simulation's origins are written (origins.cu), and the prefix
@@ -738,7 +747,7 @@ struct Engine {
     cudaGraphExec_t graph_exec = nullptr;
     std::vector<cudaEvent_t> ev_start, ev_end;
     cudaEvent_t ev_total0 = nullptr, ev_total1 = nullptr;
-    bool timing_in_graph = true;
+    bool lazy_graph = false;  // a call for one simulation: the graph is built when the run turns out long
 
     ~Engine() { release(); }
 
@@ -855,9 +864,7 @@ void setup_engine(Engine &E, const necsim_args &args, int stream_priority = 0) {
     E.args = args;
     E.device = args.device;
     CK(cudaSetDevice(E.device));
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, E.device));
-    E.n_sms = prop.multiProcessorCount;
+    CK(cudaDeviceGetAttribute(&E.n_sms, cudaDevAttrMultiProcessorCount, E.device));
     CK(cudaStreamCreateWithPriority(&E.stream, cudaStreamNonBlocking, stream_priority));
     CK(cudaStreamCreateWithPriority(&E.stream_t, cudaStreamNonBlocking, stream_priority));
     CK(cudaEventCreateWithFlags(&E.ev_fork, cudaEventDisableTiming));
@@ -909,7 +916,7 @@ void carve_run_buffers(Engine &E, Carver &c) {
     E.d_counters = c.take<SimCounters>(E.sims.size());
     E.d_ctl = c.take<Control>(1);
     E.d_spec = c.take<DevSpeciationEvent>(n);
-    E.d_disp = E.disp_cap ? c.take<DevDispersalEvent>(E.disp_cap) : nullptr;
+    E.d_disp = E.disp_room ? c.take<DevDispersalEvent>(E.disp_room) : nullptr;
 }
 
 // The run's buffers for n_cap lineages (at least n_total), as one allocation:
@@ -917,6 +924,7 @@ void carve_run_buffers(Engine &E, Carver &c) {
 void alloc_run_buffers(Engine &E, uint64_t n_cap) {
     E.n_cap = n_cap;
     E.spec_cap = n_cap;
+    E.disp_room = E.disp_cap;
     unsigned long long want = (n_cap * E.args.dedup_factor_pct + 99) / 100;
     if (want < 2) want = 2;
     unsigned long long size = 1;
@@ -940,10 +948,6 @@ void alloc_run_buffers(Engine &E, uint64_t n_cap) {
     // every round leaves the table empty
     CK(cudaMemsetAsync(E.owner, 0xff, size * sizeof(uint32_t), E.stream));
     CK(cudaMemsetAsync(E.min_gref, 0xff, size * sizeof(unsigned long long), E.stream));
-    // each run resets both; a run without lineages runs no round and reads
-    // them as they are here (upload_origins synchronises the stream next)
-    CK(cudaMemsetAsync(E.d_counters, 0, E.sims.size() * sizeof(SimCounters), E.stream));
-    CK(cudaMemsetAsync(E.d_ctl, 0, sizeof(Control), E.stream));
 }
 
 // Calls push(x, y, index, global_reference) for every origin lineage of the
@@ -1319,14 +1323,18 @@ void enqueue_rounds(Engine &E, unsigned rounds, bool events, bool external) {
 // Delivers the events of the round that just ended (dispersal reporting).
 void drain_events(Engine &E);
 
+void create_round_events(Engine &E) {
+    for (unsigned r = (unsigned)E.ev_start.size(); r < E.args.rounds_per_graph; ++r) {
+        cudaEvent_t a = nullptr, b = nullptr;
+        CK(cudaEventCreate(&a));
+        E.ev_start.push_back(a);
+        CK(cudaEventCreate(&b));
+        E.ev_end.push_back(b);
+    }
+}
+
 void build_graph(Engine &E) {
     const unsigned rounds = E.args.rounds_per_graph;
-    E.ev_start.resize(rounds);
-    E.ev_end.resize(rounds);
-    for (unsigned r = 0; r < rounds; ++r) {
-        CK(cudaEventCreate(&E.ev_start[r]));
-        CK(cudaEventCreate(&E.ev_end[r]));
-    }
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
     try {
@@ -1354,7 +1362,16 @@ struct RunResult {
 // until no simulation is active.
 RunResult run_rounds(Engine &E) {
     RunResult rr;
-    const unsigned rounds = E.args.rounds_per_graph;
+    // Rounds are enqueued in graphs of rounds_per_graph.  A call for one
+    // simulation is often over after a few rounds: it starts with short
+    // stretches of plain launches (the host is well ahead of rounds that
+    // take longer than their launches), and has a graph built once it has
+    // run for kGraphAfter rounds (capturing and instantiating one takes as
+    // long as some hundred launches).  Dispersal events leave the device
+    // round by round, two rounds at a time (survivors are in A after both).
+    constexpr uint64_t kGraphAfter = 256;
+    const unsigned graph_rounds = E.args.rounds_per_graph;
+    unsigned rounds = E.lazy_graph || E.delivery ? 2 : graph_rounds;
     CK(cudaEventRecord(E.ev_total0, E.stream));
     reset_lineages(E);
     // initial control state
@@ -1385,7 +1402,7 @@ RunResult run_rounds(Engine &E) {
     }
     CK(cudaMemcpyAsync(E.h_ctl, E.d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, E.stream));
     CK(cudaStreamSynchronize(E.stream));
-    uint64_t graph_launches = 0;
+    uint64_t enqueued = 0;
     uint64_t stalled = 0;
     unsigned long long last_steps = ~0ULL, last_live = ~0ULL;
     // one block per resident simulation, at most two per SM
@@ -1404,8 +1421,12 @@ RunResult run_rounds(Engine &E) {
         // every round advances each active simulation's horizon by at least
         // step_slice / lambda, so each live lineage expects >= step_slice
         // events per round: a valid run never reaches these bounds
-        if (++graph_launches > max_rounds / rounds + (max_rounds % rounds ? 1 : 0))
-            fail(NECSIM_E_TIMEOUT, "round limit reached (necsim_args.max_rounds)");
+        if (enqueued >= max_rounds) fail(NECSIM_E_TIMEOUT, "round limit reached (necsim_args.max_rounds)");
+        if (E.lazy_graph && !E.delivery && enqueued) {
+            rounds = (unsigned)std::min<uint64_t>(graph_rounds, enqueued);  // 2, 2, 4, 8, ...
+            if (!E.graph_exec && enqueued >= kGraphAfter) build_graph(E);
+        }
+        enqueued += rounds;
         if (E.h_ctl->steps_total == last_steps && E.h_ctl->n_cur == last_live && !res_inflight) {
             if (++stalled >= 64) fail(NECSIM_E_TIMEOUT, "no progress over 64 graph launches");
         } else {
@@ -1455,7 +1476,7 @@ RunResult run_rounds(Engine &E) {
                     CK(cudaStreamSynchronize(E.stream));
                     drain_events(E);
                 }
-            } else if (E.graph_exec && E.timing_in_graph) {
+            } else if (E.graph_exec && rounds == graph_rounds) {
                 CK(cudaGraphLaunch(E.graph_exec, E.stream));
             } else {
                 enqueue_rounds(E, rounds, true, false);
@@ -1846,6 +1867,20 @@ int guarded(necsim_ctx *ctx, char *buf, size_t cap, F &&f) {
     }
 }
 
+// The device runs Clark2Dt as AlmostInfinite with its dispersal switch.
+int32_t device_kind(int32_t k) { return k == NECSIM_ALMOST_INFINITE_CLARK2DT ? NECSIM_ALMOST_INFINITE_NORMAL : k; }
+
+// Dispersal events that the buffer of a reporting run holds: twice a round's
+// expected ones (n * per <= max(min_round_events + n, step_slice * n) per
+// simulation).
+uint64_t dispersal_room(const necsim_args &args, const std::vector<SimHost> &sims) {
+    if (!args.report_dispersal) return 0;
+    uint64_t bound = 0;
+    for (auto &sh : sims)
+        bound += std::max<uint64_t>(args.min_round_events + sh.n_origins, args.step_slice * sh.n_origins);
+    return 2 * bound + (1ULL << 20);
+}
+
 // Runs simulations (one or a batch) end to end on a fresh engine.
 void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &args,
                     const std::vector<std::vector<necsim_lineage>> *given,
@@ -1868,7 +1903,15 @@ void execute_engine(Engine &E, const necsim_reporter *reporters, bool one_report
         E.delivery = &dv;
     }
     try {
-        if (E.n_total > 0) rr = run_rounds(E);
+        if (E.n_total > 0) {
+            rr = run_rounds(E);
+        } else {
+            // no round runs: finish reads counters and control of nothing done
+            CK(cudaMemsetAsync(E.d_counters, 0, E.sims.size() * sizeof(SimCounters), E.stream));
+            CK(cudaMemsetAsync(E.d_params, 0, E.sims.size() * sizeof(SimParams), E.stream));
+            CK(cudaMemsetAsync(E.d_ctl, 0, sizeof(Control), E.stream));
+            CK(cudaStreamSynchronize(E.stream));
+        }
         finish(E, rr, reporters, one_reporter, outcomes, rem);
     } catch (...) {
         E.delivery = nullptr;
@@ -1888,8 +1931,8 @@ void run_simulations(Engine &E, std::vector<SimHost> sims, const necsim_args &ar
 void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &args,
                     const std::vector<std::vector<necsim_lineage>> *given,
                     const std::vector<SimParams> *prebuilt_tables) {
-    // the device runs Clark2Dt as AlmostInfinite with its dispersal switch
-    auto device_kind = [](int32_t k) { return k == NECSIM_ALMOST_INFINITE_CLARK2DT ? NECSIM_ALMOST_INFINITE_NORMAL : k; };
+    E.args = args;
+    E.h2d_bytes = E.d2h_bytes = 0;
     E.kind = device_kind(sims.front().sc.kind);
     for (auto &s : sims)
         if (device_kind(s.sc.kind) != E.kind) fail(NECSIM_E_UNSUPPORTED, "a batch must share one scenario kind");
@@ -1906,13 +1949,9 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
         for (auto &sh : sims) sh.noise_origins = find_noise_origins(E, sh);
     if (args.report_dispersal) {
         // every lineage stays in the global rounds, which drain the events
-        // after each round; the buffer holds twice a round's expected events
-        // (n * per <= max(min_round_events + n, step_slice * n) per simulation)
+        // after each round
         E.args.resident = 0;
-        uint64_t bound = 0;
-        for (auto &sh : sims)
-            bound += std::max<uint64_t>(args.min_round_events + sh.n_origins, args.step_slice * sh.n_origins);
-        E.disp_cap = 2 * bound + (1ULL << 20);
+        E.disp_cap = dispersal_room(args, sims);
         if (E.disp_cap * sizeof(DevDispersalEvent) > (16ULL << 30))
             fail(NECSIM_E_TOO_LARGE, "dispersal event buffer above 16 GiB (lower min_round_events or batch "
                                      "fewer simulations)");
@@ -1949,11 +1988,147 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
     // step each lineage with a whole warp on any SM (the resident kernel
     // gives a simulation one SM)
     if (E.sims.size() == 1) E.args.resident = 0;
-    choose_launch(E);
-    alloc_run_buffers(E, E.n_total);
+    if (E.arena && (E.n_cap < E.n_total || E.disp_room < E.disp_cap)) {
+        if (E.graph_exec) CK(cudaGraphExecDestroy(E.graph_exec));
+        E.graph_exec = nullptr;
+        CK(cudaFree(E.arena));
+        E.arena = nullptr;
+    }
+    if (!E.arena) {  // a fresh engine, or one that was too small
+        choose_launch(E);
+        // one simulation's workspace may serve the next call's (EnginePool):
+        // room for up to an eighth more lineages
+        uint64_t n_cap = E.n_total;
+        if (E.lazy_graph) {
+            uint64_t step = 4096;
+            while (step * 16 < n_cap) step *= 2;
+            n_cap = (n_cap + step - 1) / step * step;
+        }
+        alloc_run_buffers(E, n_cap);
+        create_round_events(E);
+    }
     upload_origins(E, given);
-    if (E.n_total > 0) build_graph(E);
+    if (E.n_total > 0 && !E.lazy_graph) build_graph(E);
 }
+
+// ---- workspaces kept between the calls of one simulation ----
+//
+// Streams, events, the pinned control word, the run buffers and the CUDA
+// graph of a finished call, for the next call of the same shape (the same
+// device, scenario kind and launch arguments, at most as many lineages):
+// setting them up and freeing them took 6 ms (a call with 1,200 lineages 7.5
+// ms, now 0.6 ms; with 100,000 lineages 11 ms, now 4.0 ms).  An
+// engine is in the pool only while no call uses it; the pool holds at most
+// kEngines engines and 1/32 of a device's memory each way, and is emptied
+// when an allocation fails.  Nothing in it depends on a call's inputs: every
+// run writes its lineages, parameters and counters anew.
+struct EnginePool {
+    static constexpr size_t kEngines = 4;
+    std::mutex mu;
+    std::vector<std::unique_ptr<Engine>> idle;
+
+    // The id of the current CUDA context (0: unknown): engines of a context
+    // that the program has reset since are forgotten, not freed.
+    static unsigned long long context_id() {
+        using GetId = int (*)(void *, unsigned long long *);
+        static const GetId get = [] {
+            void *fn = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+                q != cudaDriverEntryPointSuccess) {
+                cudaGetLastError();
+                fn = nullptr;
+            }
+            return reinterpret_cast<GetId>(fn);
+        }();
+        unsigned long long id = 0;
+        return get && get(nullptr, &id) == 0 ? id : 0;
+    }
+
+    static size_t byte_limit(int device) {
+        static std::mutex m;
+        static std::map<int, size_t> limits;
+        std::lock_guard<std::mutex> lock(m);
+        auto it = limits.find(device);
+        if (it == limits.end()) {
+            cudaDeviceProp prop;
+            CK(cudaGetDeviceProperties(&prop, device));
+            it = limits.emplace(device, prop.totalGlobalMem / 32).first;
+        }
+        return it->second;
+    }
+
+    // Arguments that an engine's buffers, launch shapes and graph depend on.
+    static bool same_shape(const Engine &E, int kind, const necsim_args &a) {
+        const necsim_args &b = E.args;
+        return E.kind == kind && a.device == E.device && a.block_size == b.block_size &&
+               a.grid_size == b.grid_size && a.dedup_factor_pct == b.dedup_factor_pct &&
+               a.rounds_per_graph == b.rounds_per_graph && a.report_dispersal == b.report_dispersal &&
+               a.event_time_sampler == b.event_time_sampler && a.schedule == 0 && b.schedule == 0;
+    }
+
+    // An idle engine with room for n lineages and disp dispersal events (the
+    // smallest one; not one with more than 8 times the room, whose buffers
+    // would be spread over memory for nothing), or null.
+    std::unique_ptr<Engine> take(int kind, const necsim_args &a, uint64_t n, uint64_t disp) {
+        const unsigned long long id = context_id();
+        std::lock_guard<std::mutex> lock(mu);
+        size_t best = idle.size();
+        for (size_t j = 0; j < idle.size(); ++j) {
+            const Engine &E = *idle[j];
+            if (id == 0 || E.context != id || !same_shape(E, kind, a) || E.n_cap < n || E.disp_room < disp) continue;
+            if (E.n_cap > 8 * std::max<uint64_t>(n, 4096)) continue;
+            if (best == idle.size() || E.n_cap < idle[best]->n_cap) best = j;
+        }
+        if (best == idle.size()) return nullptr;
+        std::unique_ptr<Engine> e = std::move(idle[best]);
+        idle.erase(idle.begin() + (std::ptrdiff_t)best);
+        return e;
+    }
+
+    void put(std::unique_ptr<Engine> e) {
+        const unsigned long long id = context_id();
+        const size_t limit = byte_limit(e->device);
+        if (id == 0 || e->args.schedule || e->arena_bytes > limit) return;
+        e->context = id;
+        std::vector<std::unique_ptr<Engine>> gone;  // freed after the lock
+        std::lock_guard<std::mutex> lock(mu);
+        for (size_t j = 0; j < idle.size();) {
+            if (idle[j]->device == e->device && idle[j]->context != id) {
+                (void)idle[j].release();  // its context is gone, and its memory with it
+                idle.erase(idle.begin() + (std::ptrdiff_t)j);
+            } else {
+                ++j;
+            }
+        }
+        size_t bytes = e->arena_bytes;
+        for (auto &o : idle) bytes += o->device == e->device ? o->arena_bytes : 0;
+        // the longest idle go first
+        while (!idle.empty() && (idle.size() >= kEngines || bytes > limit)) {
+            if (idle.front()->device == e->device) bytes -= idle.front()->arena_bytes;
+            gone.push_back(std::move(idle.front()));
+            idle.erase(idle.begin());
+        }
+        idle.push_back(std::move(e));
+    }
+
+    bool empty_out() {
+        std::vector<std::unique_ptr<Engine>> gone;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            gone.swap(idle);
+        }
+        return !gone.empty();
+    }
+};
+
+// Never destroyed: at process exit the CUDA context may be gone first.
+EnginePool &engine_pool() {
+    static EnginePool *pool = new EnginePool;
+    return *pool;
+}
+
+bool release_idle_workspaces() { return engine_pool().empty_out(); }
 
 // ---- a batch split into engines: priority simulations each run alone ----
 //
@@ -2265,29 +2440,10 @@ static int simulate_impl(necsim_ctx *ctx, const necsim_lineage *lineages, uint64
                          const necsim_reporter *reporter, necsim_outcome *outcome) {
     if (!ctx || !outcome) return NECSIM_E_INVALID_ARGUMENT;
     return guarded(ctx, nullptr, 0, [&] {
-        // a fresh engine per simulation; SE tables are carried over
-        std::unique_ptr<Engine> tables_owner;
+        // the tables stay the context's; the run's engine only reads them
         std::vector<SimParams> prebuilt;
-        Engine *E = new Engine();
-        std::unique_ptr<Engine> E_owner(E);
-        if (ctx->tables_ready) {
-            // move the table allocations into this run's engine, then back
-            Engine &T = *ctx->engine;
-            E->d_cells.swap(T.d_cells);
-            E->d_atoms.swap(T.d_atoms);
-            prebuilt.push_back(ctx->table_params);
-        }
-        struct Restore {
-            necsim_ctx *ctx;
-            Engine *E;
-            ~Restore() {
-                if (ctx->tables_ready) {
-                    ctx->engine->d_cells.swap(E->d_cells);
-                    ctx->engine->d_atoms.swap(E->d_atoms);
-                }
-            }
-        } restore{ctx, E};
-        setup_engine(*E, ctx->args);
+        if (ctx->tables_ready) prebuilt.push_back(ctx->table_params);
+        CK(cudaSetDevice(ctx->args.device));
         SimHost sh;
         std::memset(&sh, 0, sizeof(sh));
         sh.sc = ctx->scenario;
@@ -2348,9 +2504,20 @@ static int simulate_impl(necsim_ctx *ctx, const necsim_lineage *lineages, uint64
         }
         std::vector<SimHost> sims{sh};
         necsim_outcome o;
+        // (WrappingNoise counts its origins on the device: any engine may turn
+        // out too small, then it gets buffers of its own)
+        std::unique_ptr<Engine> E =
+            engine_pool().take(device_kind(sh.sc.kind), ctx->args, sh.n_origins, dispersal_room(ctx->args, sims));
+        if (!E) {
+            E.reset(new Engine());
+            setup_engine(*E, ctx->args);
+            E->lazy_graph = true;
+        }
         run_simulations(*E, sims, ctx->args, resume ? &given : nullptr, reporter, true, &o,
                         ctx->remaining, ctx->tables_ready ? &prebuilt : nullptr);
         *outcome = o;
+        E->drop_inputs();
+        engine_pool().put(std::move(E));
     });
 }
 
