@@ -893,6 +893,8 @@ void choose_launch(Engine &E) {
         if (coop_per_sm < 1) coop_per_sm = 1;
         E.coop_grid = (unsigned)(coop_per_sm * E.n_sms);
         E.coop_max = (uint64_t)E.coop_grid * (kCoopBlock / 32);
+        // a noise target takes a whole warp: every WrappingNoise round
+        if (E.kind == NECSIM_WRAPPING_NOISE) E.coop_max = ~0ULL;
     }
     E.aux_block = 256;
     E.aux_grid = (unsigned)(E.n_sms * 8);

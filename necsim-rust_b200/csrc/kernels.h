@@ -104,8 +104,8 @@ struct ScheduleArgs {
 
 // the step kernel on grid x block and, for the Poisson sampler with
 // a.coop_max > 0, the cooperative kernel on coop_grid x kCoopBlock before it
-// (a.coop_max at most coop_grid's warps); each returns at once in the
-// other's rounds
+// (a.coop_max at most coop_grid's warps; WrappingNoise: ~0, every round runs
+// in the cooperative kernel); each returns at once in the other's rounds
 cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned block, unsigned coop_grid,
                         cudaStream_t st);
 cudaError_t step_kernel_occupancy(int kind, bool exp_sampler, int block, int *blocks_per_sm);

@@ -79,6 +79,10 @@ NECSIM_NOISE_FN double rnd(double v) {
 
 // the low byte of Rust's `v as i64` (truncating, saturating, NaN -> 0)
 NECSIM_NOISE_FN uint32_t low_byte_of_i64(double v) {
+#ifdef __CUDA_ARCH__
+    // below 2^52 the integer part is the low mantissa of v + 2^52
+    if (v >= 0.0 && v < 0x1p52) return (uint32_t)__double2loint(__dadd_rz(v, 0x1p52)) & 0xffu;
+#endif
     if (v != v) return 0u;
     if (v >= 9223372036854775808.0) return 0xffu;  // i64::MAX
     if (v <= -9223372036854775808.0) return 0u;    // i64::MIN
@@ -96,8 +100,11 @@ constexpr double kFrac1Pi = 0.318309886183790671537767526745028724;  // core::f6
 // reads.  The hash reads perm[0..256) and only their low bytes:
 // (perm[a] + b) & 0xff and (perm[c] & 0x0e) >> 1 depend on nothing else.
 NECSIM_NOISE_FN double extrapolate(const uint8_t *perm, double gx, double gy, double dx, double dy, double wrap) {
-    gx = flr(sub(gx, mul(flr(div(gx, wrap)), wrap)));
-    gy = flr(sub(gy, mul(flr(div(gy, wrap)), wrap)));
+    // g - floor(g / wrap) wrap of integers: g itself in [0, wrap) (below 2^53
+    // the quotient does not round up to 1), which spares almost every call
+    // its two divisions
+    if (!(gx >= 0.0 && gx < wrap && wrap <= 0x1p53)) gx = flr(sub(gx, mul(flr(div(gx, wrap)), wrap)));
+    if (!(gy >= 0.0 && gy < wrap && wrap <= 0x1p53)) gy = flr(sub(gy, mul(flr(div(gy, wrap)), wrap)));
     const uint32_t i0 = ((uint32_t)perm[low_byte_of_i64(gx)] + low_byte_of_i64(gy)) & 0xffu;
     const uint32_t idx = ((uint32_t)perm[i0] & 0x0eu) >> 1;
     double px = (idx & 1u) == 0 ? 5.0 : 2.0;
@@ -149,13 +156,17 @@ NECSIM_NOISE_FN double eval2d(const uint8_t *perm, double x, double y, double wr
     return div(add(value, tri), 47.0);
 }
 
+// The period of octave `frequency` and the plane's scale in it.
+NECSIM_NOISE_FN double octave_period(double frequency) { return rnd(mul(kTwo32, frequency)); }
+NECSIM_NOISE_FN double first_frequency(const NoiseHabitat &h) { return mul(mul(h.scale, kFrac1Pi), 3.0); }
+
 // habitat/wrapping_noise/mod.rs:216-249 sum_noise_octaves
 NECSIM_NOISE_FN double octave_sum(const NoiseHabitat &h, uint32_t x, uint32_t y) {
     double max_amplitude = 0.0, amplitude = 1.0;
-    double frequency = mul(mul(h.scale, kFrac1Pi), 3.0);
+    double frequency = first_frequency(h);
     double result = 0.0;
     for (uint64_t o = 0; o < h.octaves; ++o) {
-        const double wrap = rnd(mul(kTwo32, frequency));  // an integer period
+        const double wrap = octave_period(frequency);
         const double fixed = mul(wrap, kTwoM32);
         result = add(result, mul(eval2d(h.perm, mul((double)x, fixed), mul((double)y, fixed), wrap), amplitude));
         max_amplitude = add(max_amplitude, amplitude);
