@@ -887,12 +887,20 @@ void choose_launch(Engine &E) {
     E.step_block = block;
     E.step_grid = E.args.grid_size ? E.args.grid_size : (unsigned)(per_sm * E.n_sms);
     if (E.args.event_time_sampler != NECSIM_SAMPLER_EXP) {
-        // one warp per lineage, all of them resident at once
+        // One warp per lineage, for rounds of up to four lineages per
+        // resident warp (9,472 with four blocks per SM).  The cooperative
+        // kernel steps about 4e9 events per second whatever the round's size
+        // (329 warp instructions per event), the step kernel, one lane per
+        // lineage, 7e9 with 30,000 live lineages of one simulation and 2 to
+        // 3e9 with 20,000 to 50,000 of many.  A limit of one / two / four /
+        // eight lineages per warp: the 64-simulation sweep takes 637 / 593 /
+        // 580 / 578 ms, with the learned schedule 516 / 502 / 499 / 509 ms,
+        // one SpatiallyImplicit run of 30,011 lineages 40 / 36 / 36 / 36 ms.
         int coop_per_sm = 0;
         CK(coop_kernel_occupancy(E.kind, &coop_per_sm));
         if (coop_per_sm < 1) coop_per_sm = 1;
         E.coop_grid = (unsigned)(coop_per_sm * E.n_sms);
-        E.coop_max = (uint64_t)E.coop_grid * (kCoopBlock / 32);
+        E.coop_max = (uint64_t)E.coop_grid * (kCoopBlock / 32) * 4;
         // a noise target takes a whole warp: every WrappingNoise round
         if (E.kind == NECSIM_WRAPPING_NOISE) E.coop_max = ~0ULL;
     }
@@ -1188,6 +1196,7 @@ StepArgs make_step_args(Engine &E, DeviceLineages &in) {
     a.order = E.learned ? E.order : nullptr;
     a.exp_sampler = E.args.event_time_sampler == NECSIM_SAMPLER_EXP ? 1u : 0u;
     a.coop_max = E.coop_max;
+    a.n_sms = (uint32_t)E.n_sms;
     // free rounds of single-lineage simulations (not when dispersal events
     // are drained round by round)
     a.free_rounds = E.args.report_dispersal ? 0u : 64u;
@@ -1210,7 +1219,7 @@ FeatureArgs make_feature_args(Engine &E, DeviceLineages &in) {
     f.params = E.d_params;
     f.counters = E.d_counters;
     f.kind = E.kind;
-    // rounds stepped one warp per lineage (the cooperative kernel, or the
+    // rounds stepped one warp at a time per lineage (the cooperative kernel, or the
     // exponential sampler's step kernel when it has a warp per lineage)
     f.skip_at_most = E.coop_max ? E.coop_max : (uint64_t)E.step_grid * (E.step_block / 32);
     return f;

@@ -1435,15 +1435,13 @@ __device__ __forceinline__ int pass_run(Lane &l, const SimParams &p, const Event
 // (or speciates) takes the next lineage of the queue, so warps stay full
 // while lineages of very different event counts drain.
 //
-// With many lineages per lane (throughput) every lane runs the same pass
-// each iteration: prime the WyHash state for either its current Poisson
-// bucket or its current event, draw samples 1..3, then take the short
-// branch for what the pass was (bucket search or event).  Lanes at
-// different points of their lineages thus execute the same instructions
-// for the hash work instead of diverging through the bucket loop, the
-// event and the refill.  With few lineages per lane (latency) each lane
-// runs lineage_step's latency form.  EXP: the exponential event-time
-// sampler, one event at a time per lane (no converged-pass form).
+// Every lane runs the same pass each iteration: prime the WyHash state for
+// either its current Poisson bucket or its current event, draw samples 1..3,
+// then take the short branch for what the pass was (bucket search or event).
+// Lanes at different points of their lineages thus execute the same
+// instructions for the hash work instead of diverging through the bucket
+// loop, the event and the refill.  EXP: the exponential event-time sampler,
+// one event at a time per lane (no converged-pass form).
 // Copies one simulation's parameters to shared memory (single-simulation
 // launches); returns the parameters the kernel reads.
 template <bool SINGLE>
@@ -1508,10 +1506,10 @@ __device__ __forceinline__ void block_arrives(const SmGate *g, uint32_t role, un
     if (g != nullptr && role != kGateNone && threadIdx.x == 0) atomicAdd(done, 1u);
 }
 
-// At most one lineage per warp: each warp takes lineages from the queue and
+// One lineage per warp at a time: each warp takes lineages from the queue and
 // steps each one with all its lanes (a lineage's events at warp latency,
-// lineages on all SMs).  Every lineage gets a warp at once, so the queue
-// order is moot (and not computed for such rounds).
+// lineages on all SMs).  At most a few lineages wait for each warp, so the
+// queue is not ordered (no order is computed for such rounds).
 template <int KIND, bool SINGLE, bool EXP>
 __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P, uint64_t n) {
     const EventSink sink = sink_of(a);
@@ -1611,7 +1609,13 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
     __shared__ __align__(16) unsigned char params_smem[SINGLE ? sizeof(SimParams) : 16];
     const uint64_t n = *a.n_cur;
     // the Poisson sampler's cooperative rounds run in coop_kernel
-    if (!EXP && n <= a.coop_max) return;
+    if (n == 0 || (!EXP && n <= a.coop_max)) return;
+    // Only the blocks that a round can fill take part: consecutive blocks sit
+    // on different SMs, while among all resident warps those of a quarter of
+    // the SMs won the race for the queue (30,000 lineages: 26.6 warps active
+    // on the busiest SM, 0.1 on the idlest).  30,000 lineages 3.5 -> 7.4e9
+    // events per second, 46,000 5.4 -> 9.8e9.
+    if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * blockDim.x >= n) return;
     if (block_leaves(a.gate, a.gate_role, a.blocks_done)) return;
     const SimParams *P = stage_params<SINGLE>(a, params_smem);
     const EventSink sink = sink_of(a);
@@ -1622,7 +1626,7 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
         block_arrives(a.gate, a.gate_role, a.blocks_done);
         return;
     }
-    const bool lat = n * 4 <= (uint64_t)gridDim.x * blockDim.x;
+    const bool lat = EXP && n * 4 <= (uint64_t)gridDim.x * blockDim.x;
     const unsigned lanemask_lt = (1u << lane_id) - 1u;
     bool have = false;
     bool exhausted = (n == 0);
@@ -1641,7 +1645,7 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
                 const unsigned long long k = base + __popc(need & lanemask_lt);
                 if (k < n) {
                     have = take_lineage<KIND, SINGLE>(a, P, k, l);
-                    if (have && !EXP && !lat && !pass_begin<KIND>(l, P[SINGLE ? 0 : l.s], ps)) {
+                    if (have && !EXP && !pass_begin<KIND>(l, P[SINGLE ? 0 : l.s], ps)) {
                         store_stopped(a, l);  // nothing to do before this horizon
                         have = false;
                     }
@@ -1657,11 +1661,13 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
         if (!have) continue;
         const SimParams &p = P[SINGLE ? 0 : l.s];
 
-        // few lineages for the grid's lanes: latency form (uniform branch);
-        // the exponential sampler steps lineages one event at a time
-        const int r = EXP ? (lat ? lineage_step<KIND, true, true>(l, p, sink)
-                                 : lineage_step<KIND, false, true>(l, p, sink))
-                          : (lat ? lineage_step<KIND, true>(l, p, sink) : pass_run<KIND>(l, p, sink, ps));
+        // the exponential sampler steps lineages one event at a time, in its
+        // latency form when there are few for the grid's lanes (uniform branch)
+        int r;
+        if constexpr (EXP)
+            r = lat ? lineage_step<KIND, true, true>(l, p, sink) : lineage_step<KIND, false, true>(l, p, sink);
+        else
+            r = pass_run<KIND>(l, p, sink, ps);
         if (r == kPassSearch) continue;
         if (r == kStepMoved) {
             local_steps += 1;
@@ -1698,17 +1704,25 @@ __global__ void __launch_bounds__(kStepBlockMax, 1) step_kernel_exp(StepArgs a) 
 }
 
 // The Poisson sampler's rounds with at most coop_max live lineages, one warp
-// per lineage (coop_run); the step kernel takes the other rounds.  Its own
-// kernel, so that the speculative form's registers do not lower the step
-// kernel's occupancy.
+// per lineage; the step kernel takes the other rounds.  Its own kernel, so
+// that the speculative form's registers do not lower the step kernel's
+// occupancy.
 template <int KIND, bool SINGLE>
 __global__ void __launch_bounds__(kCoopBlock) coop_kernel(StepArgs a) {
     __shared__ __align__(16) unsigned char params_smem[SINGLE ? sizeof(SimParams) : 16];
     const uint64_t n = *a.n_cur;
-    if (n > a.coop_max) return;
+    if (n == 0 || n > a.coop_max) return;
+    // Lineages are spread over the SMs before a second one joins a warp
+    // scheduler: one warp of a block per SM, then two, three and all four,
+    // then further blocks (consecutive blocks sit on different SMs).  The
+    // 64-simulation sweep's rounds with 145 to 754 lineages: 75 -> 51 ms.
+    const unsigned warps = a.gate_role == kGateNone && n < (uint64_t)a.n_sms * (kCoopBlock / 32)
+                               ? (unsigned)((n + a.n_sms - 1) / a.n_sms)
+                               : kCoopBlock / 32;
+    if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * warps >= n) return;
     if (block_leaves(a.gate, a.gate_role, a.blocks_done)) return;
     const SimParams *P = stage_params<SINGLE>(a, params_smem);
-    coop_body<KIND, SINGLE, false>(a, P, n);
+    if (threadIdx.x / 32u < warps) coop_body<KIND, SINGLE, false>(a, P, n);
     block_arrives(a.gate, a.gate_role, a.blocks_done);
 }
 
@@ -2185,10 +2199,6 @@ static cudaError_t launch_step_t(const StepArgs &a, unsigned grid, unsigned bloc
 
 cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned block, unsigned coop_grid,
                         cudaStream_t st) {
-    // (WrappingNoise rounds of any size run in the cooperative kernel)
-    if (!a.exp_sampler && (kind == kWrappingNoise ? a.coop_max != ~0ULL
-                                                  : a.coop_max > (uint64_t)coop_grid * (kCoopBlock / 32)))
-        return cudaErrorInvalidValue;
     switch (kind) {
     case kNonSpatial: return launch_step_t<kNonSpatial>(a, grid, block, coop_grid, st);
     case kSpatiallyImplicit: return launch_step_t<kSpatiallyImplicit>(a, grid, block, coop_grid, st);

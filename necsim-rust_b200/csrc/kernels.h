@@ -52,9 +52,10 @@ struct StepArgs {
     TraceSink trace;                     // death records of speciated lineages (tracing only)
     uint32_t exp_sampler;                // 1: exponential event-time sampler (exp.rs), else Poisson
     // Poisson sampler: rounds with at most this many live lineages run in
-    // the cooperative kernel (one warp per lineage, at most its resident
-    // warps); 0: the step kernel takes every round
+    // the cooperative kernel (one warp per lineage); 0: the step kernel takes
+    // every round (WrappingNoise: ~0, it takes none)
     uint64_t coop_max;
+    uint32_t n_sms;                      // SMs the kernels' grids are spread over
     // cooperative kernel: a simulation with one live lineage runs up to this
     // many of its next rounds in the same launch while other warps are busy
     // (or it is the launch's only simulation); 0: off.  `busy` counts the
@@ -104,8 +105,8 @@ struct ScheduleArgs {
 
 // the step kernel on grid x block and, for the Poisson sampler with
 // a.coop_max > 0, the cooperative kernel on coop_grid x kCoopBlock before it
-// (a.coop_max at most coop_grid's warps; WrappingNoise: ~0, every round runs
-// in the cooperative kernel); each returns at once in the other's rounds
+// (WrappingNoise: every round runs there); each returns at once in the
+// other's rounds
 cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned block, unsigned coop_grid,
                         cudaStream_t st);
 cudaError_t step_kernel_occupancy(int kind, bool exp_sampler, int block, int *blocks_per_sm);

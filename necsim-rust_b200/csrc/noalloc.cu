@@ -253,8 +253,9 @@ extern "C" int necsim_gpu_round_noalloc(const necsim_scenario *scenario, const n
     sa.status = reinterpret_cast<uint32_t *>(&c.ctl[kCtlStatus]);
     sa.steps_total = &c.ctl[kCtlSteps];
     sa.n_sims = 1;
+    sa.n_sms = sms;
     sa.exp_sampler = exp_sampler ? 1u : 0u;
-    sa.coop_max = exp_sampler ? 0 : (uint64_t)coop_grid * (kCoopBlock / 32);
+    sa.coop_max = exp_sampler ? 0 : (uint64_t)coop_grid * (kCoopBlock / 32) * 4;
     if (launch_step(scenario->kind, sa, step_grid, kBlock, coop_grid, st) != cudaSuccess) return NECSIM_E_CUDA;
 
     DedupArgs da;

@@ -106,3 +106,19 @@ def test_pause_and_dispersal_events(nb, syn, oracle, name, pause):
     rem, crem = np.sort(g.remaining, order="gref"), np.sort(c.remaining, order="gref")
     for f in ("gref", "x", "y", "index", "last_event_time"):
         assert np.array_equal(rem[f], crem[f]), f
+
+
+@pytest.mark.parametrize("n", [147, 148, 149, 296, 297, 592, 593, 2368, 2369, 9471, 9472, 9473, 9600, 18944, 18945])
+@pytest.mark.parametrize("kind", [0, 2])
+def test_round_sizes(nb, syn, oracle, n, kind):
+    """Lineage counts at the edges of the warps, blocks and kernels that take
+    a round (148 SMs, four warps per block, four lineages per resident warp)."""
+    if kind == 0:
+        desc = ns(n, 1, 1, 0.05)
+    else:
+        desc = dict(kind=2, speciation_probability=0.05, sigma=2.0, sample=(7, 9, n, 1))
+    with nb.Simulation(syn.to_scenario(desc), 0.05, nb.CUDA(step_slice=2, min_round_events=1)) as sim:
+        g = sim.simulate(5)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice_max=1024, step_slice=2, min_round_events=1)
+    assert same_stream(g.speciation, c.speciation)
+    assert (g.steps, g.n_rounds, g.n_dedup, g.time) == (c.steps, c.n_rounds, c.n_dedup, c.time)
