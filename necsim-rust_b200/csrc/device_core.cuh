@@ -453,7 +453,7 @@ __device__ __forceinline__ void clamp_round_dispersal(uint32_t x, uint32_t y, do
 // pow_fast_one (:167-189) from samples 2 (u01, [0, 1)) and 3 (angle, (0, 1]):
 // jump = sqrt(u * (pow(1 / (1 - u01), 1 / p) - 1)), theta = u2 * 2 * pi,
 // displacement (cos(theta) * jump, sin(theta) * jump).  The transcendental
-// calls are CUDA's f64 pow/cos/sin; their results only pass through
+// calls are CUDA's f64 pow and sincos; their results only pass through
 // round(), like the Normal sampler's.
 __device__ __forceinline__ void clark2dt_displacement(uint64_t d0, uint64_t d1, double shape_u, double exponent,
                                                       double &dx, double &dy) {
@@ -463,8 +463,10 @@ __device__ __forceinline__ void clark2dt_displacement(uint64_t d0, uint64_t d1, 
     const double powed = exponent == 1.0 ? base : pow(base, exponent);
     const double jump = __dsqrt_rn(__dmul_rn(shape_u, __dsub_rn(powed, 1.0)));
     const double theta = __dmul_rn(__dmul_rn(u2, 2.0), 3.141592653589793);
-    dx = __dmul_rn(cos(theta), jump);
-    dy = __dmul_rn(sin(theta), jump);
+    double s, c;
+    sincos(theta, &s, &c);
+    dx = __dmul_rn(c, jump);
+    dy = __dmul_rn(s, jump);
 }
 
 __device__ __forceinline__ void clark2dt_dispersal_draw(uint64_t d0, uint64_t d1, double shape_u,
@@ -477,15 +479,17 @@ __device__ __forceinline__ void clark2dt_dispersal_draw(uint64_t d0, uint64_t d1
 
 // rng.rs:180-197 sample_2d_normal (Box-Muller) scaled by sigma
 // (almost_infinite_normal.rs:58-68) from the two samples, with CUDA's f64
-// log/sin/cos
+// log and sincos
 __device__ __forceinline__ void normal_displacement(uint64_t d0, uint64_t d1, double sigma, double &dx,
                                                     double &dy) {
     const double u0 = unit_open_closed(d0);
     const double u1 = unit_closed_open(d1);
     const double r = __dsqrt_rn(__dmul_rn(-2.0, log(u0)));
     const double theta = __dmul_rn(-kTau, u1);
-    const double z0 = __dmul_rn(r, sin(theta));
-    const double z1 = __dmul_rn(r, cos(theta));
+    double s, c;
+    sincos(theta, &s, &c);  // the bits of sin and cos (2^26 angles compared), one range reduction
+    const double z0 = __dmul_rn(r, s);
+    const double z1 = __dmul_rn(r, c);
     dx = __dadd_rn(__dmul_rn(z0, sigma), 0.0);
     dy = __dadd_rn(__dmul_rn(z1, sigma), 0.0);
 }

@@ -962,9 +962,10 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
 //    with the event computed.
 // Measured with one lineage on a B200 (1,965 MHz), coop_run -> chain_run:
 // NonSpatial 1,772 -> 673 cycles per event, SpatiallyImplicit 1,747 -> 663,
-// AlmostInfinite Normal 2,793 -> 1,892, Clark2Dt 3,376 -> 2,568.  The bound
-// is the instruction count: a lone warp issues one instruction every two
-// cycles, and NonSpatial takes 329 per event (48 a prime, 31 a sample).
+// AlmostInfinite Normal 2,793 -> 1,503, Clark2Dt 3,376 -> 2,173 (1,892 and
+// 2,568 with separate sin and cos).  The bound is the instruction count: a
+// lone warp issues one instruction every two cycles, and NonSpatial takes 329
+// per event (48 a prime, 31 a sample), AlmostInfinite Normal 524.
 template <int KIND>
 constexpr bool kChainKind = KIND == kNonSpatial || KIND == kSpatiallyImplicit || KIND == kAlmostInfiniteNormal;
 
