@@ -15,7 +15,7 @@ LIB = os.path.join(LIB_DIR, "libnecsim_b200.so")
 DRIVER = os.path.join(LIB_DIR, "necsim-b200")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CU_SOURCES = ["kernels.cu", "origins.cu", "noalloc.cu", "learned.cu"]
+CU_SOURCES = ["kernels.cu", "origins.cu", "sort.cu", "noalloc.cu", "learned.cu"]
 CPP_SOURCES = ["host.cpp", "tables.cpp", "event_log.cpp", "maps.cpp"]
 DRIVER_SOURCES = ["driver.cpp", "ron.cpp"]
 
