@@ -646,6 +646,7 @@ struct DeviceLineages {
 
 struct Control {  // small device scalars
     unsigned long long n_cur, out_count, work, mask, n_spec_total, n_disp_total, steps_total, visits;
+    unsigned long long rounds_seen;  // the most rounds that a simulation has begun
     unsigned int n_active;    // active simulations in the global rounds
     uint32_t status;
     unsigned int n_resident;  // active simulations owned by the resident kernel
@@ -716,6 +717,7 @@ struct Engine {
     unsigned coop_grid = 0;   // cooperative kernel (Poisson sampler), kCoopBlock threads per block
     uint64_t coop_max = 0;    // rounds with at most this many live lineages run there
     unsigned aux_grid = 0, aux_block = 256;
+    uint32_t slice = 0;  // events of a lineage per launch of the step kernel (StepArgs)
 
     // SM reservation between the engines of a batch (owned by the batch):
     // kGateOnly for the priority engine, which turns it on once its live
@@ -912,6 +914,16 @@ void choose_launch(Engine &E) {
     }
     E.aux_block = 256;
     E.aux_grid = (unsigned)(E.n_sms * 8);
+    // Simulations of a batch are at rounds of very different lengths (10 to
+    // 1,024 events per lineage by default).  Unsliced, a launch of the step
+    // kernel lasts as long as its longest lineage, at 4 us per event, and
+    // simulations with short rounds wait: 47 rounds of the 64-simulation
+    // sweep took 4 to 8 ms each with the device mostly idle.  At most 0 (all)
+    // / 32 / 64 / 128 / 256 events per launch: 583 / 540 / 511 / 519 / 518
+    // ms, with the learned schedule 526 / 509 / 475 / 478 / 487 and 489 / 522
+    // / 495 / 474 / 460 (two seeds).  Traces and dispersal events are
+    // collected round by round.
+    if (E.sims.size() > 1 && !E.tracing && !E.args.report_dispersal) E.slice = 128;
 }
 
 void carve_run_buffers(Engine &E, Carver &c) {
@@ -1202,6 +1214,7 @@ StepArgs make_step_args(Engine &E, DeviceLineages &in) {
     a.order = E.learned ? E.order : nullptr;
     a.exp_sampler = E.args.event_time_sampler == NECSIM_SAMPLER_EXP ? 1u : 0u;
     a.coop_max = E.coop_max;
+    a.slice = E.slice;
     a.n_sms = (uint32_t)E.n_sms;
     // free rounds of single-lineage simulations (not when dispersal events
     // are drained round by round)
@@ -1276,6 +1289,7 @@ ResidentArgs make_resident_args(Engine &E, uint32_t budget, const int *stop_flag
     a.steps_total = &E.d_ctl->steps_total;
     a.visits = &E.d_ctl->visits;
     a.n_resident = &E.d_ctl->n_resident;
+    a.rounds_seen = &E.d_ctl->rounds_seen;
     a.stop_flag = stop_flag;
     a.exp_sampler = E.args.event_time_sampler == NECSIM_SAMPLER_EXP ? 1u : 0u;
     a.gate = E.gate;
@@ -1301,6 +1315,7 @@ ScheduleArgs make_schedule_args(Engine &E) {
     a.visits = &E.d_ctl->visits;
     a.n_resident = &E.d_ctl->n_resident;
     a.blocks_done = &E.d_ctl->blocks_done;
+    a.rounds_seen = &E.d_ctl->rounds_seen;
     return a;
 }
 
@@ -1438,7 +1453,7 @@ RunResult run_rounds(Engine &E) {
         // every round advances each active simulation's horizon by at least
         // step_slice / lambda, so each live lineage expects >= step_slice
         // events per round: a valid run never reaches these bounds
-        if (enqueued >= max_rounds) fail(NECSIM_E_TIMEOUT, "round limit reached (necsim_args.max_rounds)");
+        if (E.h_ctl->rounds_seen > max_rounds) fail(NECSIM_E_TIMEOUT, "round limit reached (necsim_args.max_rounds)");
         if (E.lazy_graph && !E.delivery && enqueued) {
             rounds = (unsigned)std::min<uint64_t>(graph_rounds, enqueued);  // 2, 2, 4, 8, ...
             if (!E.graph_exec && enqueued >= kGraphAfter) build_graph(E);

@@ -129,7 +129,8 @@ __device__ __forceinline__ bool spatially_explicit_dispersal_draw(
 }  // namespace
 
 // Where an event left the lineage.
-enum StepResult : int { kStepStop = 0, kStepMoved = 1, kStepSpeciated = 2, kStepDropped = 3 };
+// (kStepSlice: short of the horizon, the launch's events executed)
+enum StepResult : int { kStepStop = 0, kStepMoved = 1, kStepSpeciated = 2, kStepDropped = 3, kStepSlice = 5 };
 
 // Outputs of lineage_step besides the lineage itself.
 struct EventSink {
@@ -1366,6 +1367,17 @@ __device__ __forceinline__ void store_stopped(const StepArgs &a, const Lane &l) 
     a.in.has_next[l.slot] = 1;
 }
 
+// Keeps a lineage that stopped short of the horizon after an event.
+__device__ __forceinline__ void store_sliced(const StepArgs &a, const Lane &l) {
+    a.in.x[l.slot] = l.x;
+    a.in.y[l.slot] = l.y;
+    a.in.idx[l.slot] = l.i;
+    a.in.last[l.slot] = l.last;
+    a.in.steps[l.slot] = l.steps;
+    a.in.has_next[l.slot] = 0;
+    a.counters[l.s].unfinished = 1;
+}
+
 // A lane's lineage in converged passes: the pass kind, the current Poisson
 // bucket, the time the search starts after, and the location term.
 struct Pass {
@@ -1533,10 +1545,15 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
         const NoiseLane noise_lanes = noise_lane<KIND>(p);
         int r;
         if constexpr (EXP) {
+            uint32_t moved = 0;
             for (;;) {
                 r = lineage_step_coop<KIND, true>(c, p, sink, noise_lanes);
                 if (r != kStepMoved) break;
                 warp_steps += 1;
+                if (++moved == a.slice) {
+                    r = kStepSlice;
+                    break;
+                }
             }
             if (r == kStepSpeciated) warp_steps += 1;
         } else {
@@ -1597,6 +1614,8 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
         if (lane_id == 0) {
             if (r == kStepStop)
                 store_stopped(a, c);
+            else if (r == kStepSlice)
+                store_sliced(a, c);
             else
                 a.state[c.slot] = (r == kStepSpeciated) ? 1 : 2;
         }
@@ -1633,6 +1652,7 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
     bool exhausted = (n == 0);
     Lane l;
     uint64_t local_steps = 0;
+    uint32_t moved = 0;  // events of the lane's lineage in this launch
     Pass ps;  // converged form
 
     for (;;) {
@@ -1646,6 +1666,7 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
                 const unsigned long long k = base + __popc(need & lanemask_lt);
                 if (k < n) {
                     have = take_lineage<KIND, SINGLE>(a, P, k, l);
+                    moved = 0;
                     if (have && !EXP && !pass_begin<KIND>(l, P[SINGLE ? 0 : l.s], ps)) {
                         store_stopped(a, l);  // nothing to do before this horizon
                         have = false;
@@ -1672,9 +1693,9 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
         if (r == kPassSearch) continue;
         if (r == kStepMoved) {
             local_steps += 1;
-            continue;
-        }
-        if (r == kStepStop) {
+            if (++moved != a.slice) continue;
+            store_sliced(a, l);
+        } else if (r == kStepStop) {
             store_stopped(a, l);  // keep the peeked time for the next round
         } else {
             if (r == kStepSpeciated) local_steps += 1;
@@ -1958,6 +1979,8 @@ __global__ void __launch_bounds__(THREADS, 1) resident_kernel(ResidentArgs a) {
                 if (next_horizon(pm, n, h)) {
                     pm.horizon = h;
                     c.n_rounds += 1;
+                    if (c.n_rounds > *(volatile const unsigned long long *)a.rounds_seen)
+                        atomicMax(a.rounds_seen, c.n_rounds);
                     s_h = h;
                     s_go = 1;
                     // the global rounds running beside this launch have
@@ -2015,6 +2038,10 @@ __global__ void dedup_insert_kernel(DedupArgs a) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n;
          j += (uint64_t)gridDim.x * blockDim.x) {
         if (a.state[j] != 0) continue;
+        if (a.counters[a.in.sim[j]].unfinished) {  // its round goes on: nothing merges yet
+            a.slot[j] = kEmpty;
+            continue;
+        }
         uint64_t h = dedup_hash(a.in.sim[j], a.in.x[j], a.in.y[j], a.in.idx[j], a.in.last[j]) & mask;
         uint32_t slot = kEmpty;
         for (uint64_t probe = 0; probe <= mask; ++probe) {
@@ -2071,7 +2098,8 @@ __global__ void dedup_compact_kernel(DedupArgs a) {
         // kResidentMax lineages move to its segment of the resident arena
         // (the resident kernel owns the simulation from the next round on)
         const bool to_arena = survivor && a.arena.x != nullptr &&
-                              a.counters[s].n_live <= (unsigned long long)a.resident_max;
+                              a.counters[s].n_live <= (unsigned long long)a.resident_max &&
+                              a.counters[s].unfinished == 0;
         const bool to_out = survivor && !to_arena;
         const unsigned sv = __ballot_sync(kFull, to_out);
         unsigned long long dst_base = 0;
@@ -2170,8 +2198,13 @@ __global__ void schedule_kernel(ScheduleArgs a) {
         SimCounters &c = a.counters[s];
         if (p.resident) continue;  // the resident kernel schedules it
         const unsigned long long live = c.n_live_next;
-        c.n_live = live;
         c.n_live_next = 0;
+        if (c.unfinished) {  // the same round again
+            c.unfinished = 0;
+            my_active += 1;
+            continue;
+        }
+        c.n_live = live;
         double h;
         const bool more = next_horizon(p, live, h);
         const unsigned long long now = global_ns();
@@ -2181,6 +2214,8 @@ __global__ void schedule_kernel(ScheduleArgs a) {
         if (more) {
             p.horizon = h;
             c.n_rounds += 1;
+            if (a.rounds_seen && c.n_rounds > *(volatile const unsigned long long *)a.rounds_seen)
+                atomicMax(a.rounds_seen, c.n_rounds);
         }
         p.active = more ? 1 : 0;
         if (c.routed) {

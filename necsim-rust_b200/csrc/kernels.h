@@ -56,6 +56,11 @@ struct StepArgs {
     // every round (WrappingNoise: ~0, it takes none)
     uint64_t coop_max;
     uint32_t n_sms;                      // SMs the kernels' grids are spread over
+    // Batches: the step kernel runs at most this many events of a lineage in
+    // a launch (0: all up to the horizon); a simulation with a lineage left
+    // short of its horizon goes on in the next launch, without merging, and
+    // its round ends in the launch that leaves none
+    uint32_t slice;
     // cooperative kernel: a simulation with one live lineage runs up to this
     // many of its next rounds in the same launch while other warps are busy
     // (or it is the launch's only simulation); 0: off.  `busy` counts the
@@ -101,6 +106,7 @@ struct ScheduleArgs {
     unsigned long long *visits;          // lineages the scheduled rounds process
     unsigned int *n_resident;            // active simulations owned by the resident kernel
     unsigned int *blocks_done;           // the next round's kernel arrivals (reset here)
+    unsigned long long *rounds_seen;     // the most rounds that a simulation has begun
 };
 
 // the step kernel on grid x block and, for the Poisson sampler with
@@ -127,6 +133,7 @@ struct ResidentArgs {
     unsigned long long *steps_total;
     unsigned long long *visits;
     unsigned int *n_resident;
+    unsigned long long *rounds_seen;     // the most rounds that a simulation has begun
     const int *stop_flag;                // set when the concurrent global rounds end (nullable)
     uint32_t exp_sampler;                // 1: exponential event-time sampler (exp.rs), else Poisson
     const SmGate *gate;                  // SM reservation (nullable) and this engine's role in it

@@ -153,6 +153,9 @@ struct SimCounters {
     unsigned long long n_live_next;    // survivors of the current round
     unsigned long long n_dispersal;
     unsigned long long routed;         // survivors were moved to the resident arena
+    // a lineage stopped short of the horizon (StepArgs.slice): the round goes
+    // on in the next launch, its lineages are not merged yet
+    unsigned long long unfinished;
     // device clock (%globaltimer, ns): the simulation's first schedule, its
     // hand-over to the resident kernel (0: never) and its end or pause
     unsigned long long start_ns, routed_ns, end_ns;
