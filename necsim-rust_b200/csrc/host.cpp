@@ -530,6 +530,7 @@ bool chain_scenario(const SimParams &p, int32_t kind) {
     case NECSIM_SPATIALLY_IMPLICIT:
         return (uint64_t)p.width * p.height <= most && (uint64_t)p.meta_width * p.meta_height <= most &&
                (p.meta_ox > p.width - 1 || p.meta_oy > p.height - 1);
+    case NECSIM_SPATIALLY_EXPLICIT: return (uint64_t)p.width * p.height <= most;
     case NECSIM_ALMOST_INFINITE_NORMAL:
     case NECSIM_ALMOST_INFINITE_CLARK2DT: return true;
     default: return false;

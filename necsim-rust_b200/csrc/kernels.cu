@@ -937,10 +937,9 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
     }
 }
 
-// ---- the cooperative step of the scenarios without tables ----
+// ---- the cooperative step for one lineage's latency ----
 //
-// chain_run is coop_run for NonSpatial, SpatiallyImplicit and AlmostInfinite
-// (the same lane roles, the same results), written for the latency of the
+// chain_run is coop_run (the same lane roles, the same results), written for the latency of the
 // one dependent chain that every tail is:
 //  * the lineage is its location term, its time bucket and its last event
 //    time in units of delta_t (a power of two: every product with it is
@@ -964,11 +963,12 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
 // Measured with one lineage on a B200 (1,965 MHz), coop_run -> chain_run:
 // NonSpatial 1,772 -> 673 cycles per event, SpatiallyImplicit 1,747 -> 663,
 // AlmostInfinite Normal 2,793 -> 1,503, Clark2Dt 3,376 -> 2,173 (1,892 and
-// 2,568 with separate sin and cos).  The bound is the instruction count: a
+// 2,568 with separate sin and cos), SpatiallyExplicit 3,019 -> 2,341 (64 x 64
+// map; its atoms, 190 MB, come from HBM).  The bound is the instruction count: a
 // lone warp issues one instruction every two cycles, and NonSpatial takes 329
 // per event (48 a prime, 31 a sample), AlmostInfinite Normal 524.
 template <int KIND>
-constexpr bool kChainKind = KIND == kNonSpatial || KIND == kSpatiallyImplicit || KIND == kAlmostInfiniteNormal;
+constexpr bool kChainKind = KIND != kWrappingNoise;
 
 // Whether chain_run takes the simulation's round: SimParams.chain (delta_t a
 // power of two, every table length below 2^32, no metacommunity cell inside
@@ -1022,11 +1022,17 @@ __device__ __forceinline__ Community community_of(const SimParams &p, bool local
 }
 
 // The coordinates of a location term (the inverse of location_term and
-// injection_at).
+// injection_at); `map_cell`: the cell of a SpatiallyExplicit location.
 template <int KIND>
-__device__ __forceinline__ void chain_unpack(const SimParams &p, uint64_t loc_term, bool local, uint32_t &x,
-                                             uint32_t &y, uint32_t &i) {
+__device__ __forceinline__ void chain_unpack(const SimParams &p, uint64_t loc_term, bool local, uint32_t map_cell,
+                                             uint32_t &x, uint32_t &y, uint32_t &i) {
     const uint64_t inj = seahash_undiffuse(swap_halves(loc_term ^ (p.seed ^ kWyP0)));
+    if (KIND == kSpatiallyExplicit) {
+        y = map_cell / p.width;
+        x = map_cell - y * p.width;
+        i = (uint32_t)(inj - p.cells[map_cell].injection);
+        return;
+    }
     if (KIND == kAlmostInfiniteNormal) {
         x = (uint32_t)inj;
         y = (uint32_t)(inj >> 32);
@@ -1049,6 +1055,8 @@ struct Chain {
     double before;       // the search's start, in units of delta_t
     double next;         // peeked event time, in units of delta_t
     uint32_t x, y;       // AlmostInfinite
+    uint32_t cell;       // SpatiallyExplicit: the cell, in range, and
+    CellRecord rec;      // its record
     uint32_t moved;      // events executed
     bool peek;           // `next` and `reprime` hold a peeked event
     bool local;          // SpatiallyImplicit: in the local community
@@ -1080,8 +1088,16 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
     const uint64_t seed_term = p.seed ^ kWyP0;
     // X > t  <=>  d > t 2^11 + 2047 for X = d >> 11 (never for t >= 2^53 - 1)
     auto above = [](uint64_t t) { return t >= (1ULL << 53) - 1 ? ~0ULL : (t << 11) | 2047ULL; };
-    const uint64_t more0 = above(p.pois.threshold[0]), more1 = above(p.pois.threshold[1]),
-                   more2 = above(p.pois.threshold[2]), more3 = above(p.pois.threshold[3]);
+    uint64_t more0, more1, more2, more3;
+    const PoissonConsts *pc = &p.pois;
+    auto sampler_here = [&] {  // (per cell under a turnover map)
+        if (KIND == kSpatiallyExplicit && p.turnover_cells) pc = &p.turnover_cells[c.cell];
+        more0 = above(pc->threshold[0]);
+        more1 = above(pc->threshold[1]);
+        more2 = above(pc->threshold[2]);
+        more3 = above(pc->threshold[3]);
+    };
+    sampler_here();
     // X < t  <=>  d <= t 2^11 - 1 for 0 < t <= 2^53
     const uint64_t leave_at_most = ((kMigrates ? p.migration_threshold : p.nu_threshold) << 11) - 1ULL;
     // floor(u L) = floor(X (L 2^-53)): the scaling is exact, so the product
@@ -1108,7 +1124,8 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
     enter();
     for (;;) {
         uint64_t s, d1, loc_next;
-        uint32_t sel, tx = 0, ty = 0;
+        uint32_t sel, tx = 0, ty = 0;  // SpatiallyExplicit: tx is the target's cell
+        uint32_t err = 0;              // SpatiallyExplicit: status bits of a failed bound check
         double mine;
         bool leave;
         for (;;) {
@@ -1130,6 +1147,39 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
                 else
                     normal_dispersal_draw(d2, d3, sigma, c.x, c.y, tx, ty);
                 inj_k = (((uint64_t)ty << 32) | (uint64_t)tx) * kSeaHashK;
+            } else if constexpr (KIND == kSpatiallyExplicit) {
+                // packed_separable_alias/dispersal.rs:16-77 (the cases of
+                // spatially_explicit_dispersal_draw): each lane reads its own
+                // candidate's alias atom and target record, while the search
+                // is decided (read after the selection an event took 3,019 cycles)
+                const double sd = c.rec.self_dispersal;
+                const bool stays = sd == 1.0, plain = sd == 0.0 || c.rec.non_self_event != c.cell;
+                const bool alias = !stays && (plain || __dmul_rn(v2, 0x1p-53) >= sd);
+                const double va = plain ? v2 : v3;
+                const double vc = stays ? v2 : (plain || !alias ? v3 : v4);
+                uint32_t target = c.cell;
+                err = 0;
+                if (alias) {
+                    const double f = __dmul_rn(va, __dmul_rn(__uint2double_rn(c.rec.atom_count), 0x1p-53));
+                    const uint32_t at_cell = floor_u32(f);
+                    const double frac = __dsub_rn(f, exact_double(at_cell));
+                    const uint64_t at = (uint64_t)c.rec.atom_start + at_cell;
+                    if (at_cell >= c.rec.atom_count || at >= p.n_atoms) {
+                        err = kErrAtomIndex;
+                    } else {
+                        const AliasAtom atom = p.atoms[at];
+                        target = frac < atom.u ? atom.e : atom.k;
+                    }
+                }
+                inj_k = 0;
+                if (target >= p.n_cells) err |= kErrCellIndex;
+                if (err == 0) {
+                    const CellRecord &there = p.cells[target];
+                    const double habitat_u = __dmul_rn(exact_double(there.habitat), 0x1p-53);
+                    inj_k = (there.injection + floor_u32(__dmul_rn(vc, habitat_u))) * kSeaHashK;
+                }
+                tx = target;
+                leave = leave || err != 0;
             } else {
                 const uint32_t cell = floor_u32(__dmul_rn(kMigrates ? v3 : v2, cells_u));
                 const uint32_t i = floor_u32(__dmul_rn(kMigrates ? v4 : v3, deme_u));
@@ -1170,6 +1220,11 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
                 c.x = __shfl_sync(kFull, tx, (int)sel);
                 c.y = __shfl_sync(kFull, ty, (int)sel);
             }
+            if (KIND == kSpatiallyExplicit) {
+                c.cell = __shfl_sync(kFull, tx, (int)sel);
+                c.rec = p.cells[c.cell];
+                if (p.turnover_cells) sampler_here();
+            }
             c.loc_term = ((uint64_t)hi << 32) | lo;
             tk += (uint64_t)(sel >> 28) * kSeaHashK;
             start_bits += sel >> 28;
@@ -1195,7 +1250,7 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
                 // with events at lambda delta_t = 1): lane j draws j, j + 32, ...
                 const uint64_t s_b = __shfl_sync(kFull, s, (int)b_sel), d1_b = __shfl_sync(kFull, d1, (int)b_sel);
                 const double start_b = exact_double(c.base + b_sel);
-                const uint32_t n_ev = poisson_count(d1_b, p.pois);
+                const uint32_t n_ev = poisson_count(d1_b, *pc);
                 long long best = kNoEvent;
                 uint32_t best_k = 0xffffffffu;
                 for (uint32_t j = lane; j < n_ev; j += 32u) {
@@ -1236,8 +1291,15 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
         }
         c.peek = false;
         const bool leaves = __shfl_sync(kFull, leave ? 1 : 0, (int)cand) != 0;
+        if (KIND == kSpatiallyExplicit && leaves) {
+            // a speciation, or a bound check that failed
+            if (__shfl_sync(kFull, d1 <= leave_at_most ? 1 : 0, (int)cand)) return kStepSpeciated;
+            const uint32_t bits = __shfl_sync(kFull, err, (int)cand);
+            if (lane == 0) set_status(k.status, bits);
+            return kStepDropped;
+        }
         if (leaves && !kMigrates) return kStepSpeciated;
-        if (k.report_dispersal && lane == 0) chain_unpack<KIND>(p, c.loc_term, LOCAL, l.x, l.y, l.i);
+        if (k.report_dispersal && lane == 0) chain_unpack<KIND>(p, c.loc_term, LOCAL, c.cell, l.x, l.y, l.i);
         if (leaves) {
             // migration: the target in the metacommunity from samples 3 and 4
             const uint64_t s_e = __shfl_sync(kFull, s, (int)cand);
@@ -1251,10 +1313,15 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
             c.loc_term = __shfl_sync(kFull, loc_next, (int)cand);
             c.x = __shfl_sync(kFull, tx, (int)cand);
             c.y = __shfl_sync(kFull, ty, (int)cand);
+            if (KIND == kSpatiallyExplicit) {
+                c.cell = c.x;
+                c.rec = p.cells[c.cell];
+                sampler_here();
+            }
         }
         if (k.report_dispersal && lane == 0) {
             uint32_t ex, ey, ei;
-            chain_unpack<KIND>(p, c.loc_term, LOCAL && !leaves, ex, ey, ei);
+            chain_unpack<KIND>(p, c.loc_term, LOCAL && !leaves, c.cell, ex, ey, ei);
             l.next = __dmul_rn(c.next, p.delta_t);
             emit_dispersal(l, k, ex, ey, ei);
             l.last = l.next;
@@ -1284,6 +1351,10 @@ __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const Even
     c.peek = l.has_next;
     c.x = l.x;
     c.y = l.y;
+    if (KIND == kSpatiallyExplicit) {
+        c.cell = l.y * p.width + l.x;  // below 2^32 (SimParams.chain) and in the table: l.rec was read there
+        c.rec = l.rec;
+    }
     c.moved = 0;
     c.local = KIND != kSpatiallyImplicit || in_local(p, l.x, l.y);
     const uint64_t steps = l.steps;
@@ -1300,7 +1371,8 @@ __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const Even
     l.next = __dmul_rn(c.next, p.delta_t);
     l.reprime = c.reprime;
     l.has_next = result == kStepStop;
-    chain_unpack<KIND>(p, c.loc_term, c.local, l.x, l.y, l.i);
+    chain_unpack<KIND>(p, c.loc_term, c.local, c.cell, l.x, l.y, l.i);
+    if (KIND == kSpatiallyExplicit) l.rec = c.rec;
     if (result == kStepSpeciated && (threadIdx.x & 31u) == 0u) emit_speciation(l, k);
     return result;
 }

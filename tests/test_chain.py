@@ -122,3 +122,75 @@ def test_round_sizes(nb, syn, oracle, n, kind):
     c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice_max=1024, step_slice=2, min_round_events=1)
     assert same_stream(g.speciation, c.speciation)
     assert (g.steps, g.n_rounds, g.n_dedup, g.time) == (c.steps, c.n_rounds, c.n_dedup, c.time)
+
+
+def se(syn, w, h, sigma, nu, cell=12, p_zero=0.2, dispersal=None, seed=3, **kw):
+    hab = syn.habitat_map(w, h, p_zero, cell, seed)
+    hab.flat[0] = max(1, hab.flat[0])
+    disp = syn.dispersal_map(hab, sigma) if dispersal is None else dispersal(hab)
+    return dict(kind=3, speciation_probability=nu, width=w, height=h, habitat=hab, dispersal=disp, **kw)
+
+
+def only_self(hab):
+    return np.diag((hab.reshape(-1) > 0).astype(np.float64))
+
+
+def never_self(hab):
+    d = np.tile((hab.reshape(-1) > 0).astype(np.float64), (hab.size, 1))
+    np.fill_diagonal(d, 0.0)
+    d[hab.reshape(-1) == 0] = 0.0
+    return d
+
+
+SE_CASES = {
+    # name: (scenario, kernel arguments)
+    "one_cell": (lambda syn: se(syn, 1, 1, 1.0, 0.02, p_zero=0.0), {}),
+    "one_row": (lambda syn: se(syn, 23, 1, 1.0, 0.01), {}),
+    "self_only": (lambda syn: se(syn, 7, 5, 1.0, 0.01, dispersal=only_self), {}),
+    "self_never": (lambda syn: se(syn, 7, 5, 1.0, 0.01, dispersal=never_self), {}),
+    "narrow": (lambda syn: se(syn, 11, 9, 0.3, 0.01), {}),
+    "many_events_per_bucket": (lambda syn: se(syn, 11, 9, 2.0, 0.005), dict(delta_t=16.0)),
+    "few_events_per_bucket": (lambda syn: se(syn, 11, 9, 2.0, 0.02), dict(delta_t=0.125)),
+    "delta_t_no_power_of_two": (lambda syn: se(syn, 11, 9, 2.0, 0.005), dict(delta_t=3.0)),
+    "short_rounds": (lambda syn: se(syn, 11, 9, 2.0, 0.01), dict(step_slice=1, min_round_events=1)),
+    "every_event_speciates": (lambda syn: se(syn, 5, 4, 2.0, 1.0), {}),
+    "turnover_map": (lambda syn: se(syn, 11, 9, 2.0, 0.005,
+                                    turnover_map=0.1 + 3.0 * syn.unit(9, 99, 4).reshape(9, 11)), {}),
+}
+
+
+@pytest.mark.parametrize("name", sorted(SE_CASES))
+@pytest.mark.parametrize("batch", [False, True])
+def test_explicit_matches_oracle(nb, syn, oracle, name, batch):
+    """SpatiallyExplicit: every candidate reads its own alias atom and record."""
+    make, kw = SE_CASES[name]
+    desc = make(syn)
+    nu = desc["speciation_probability"]
+    if batch:
+        g = nb.simulate_batch([syn.to_scenario(desc)] * 2, [nu, min(1.0, 2 * nu)], [5, 6],
+                              nb.CUDA(resident=True, **kw), collect=True)[0]
+    else:
+        with nb.Simulation(syn.to_scenario(desc), nu, nb.CUDA(**kw)) as sim:
+            g = sim.simulate(5)
+    oracle_kw = dict(dict(step_slice=10, min_round_events=1 << 20), **kw)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice_max=1024, **oracle_kw)
+    assert g.steps == c.steps > 0
+    assert same_stream(g.speciation, c.speciation)
+    assert (g.n_rounds, g.n_dedup, g.time) == (c.n_rounds, c.n_dedup, c.time)
+
+
+def test_explicit_dispersal_events(nb, syn, oracle):
+    desc = se(syn, 11, 9, 1.0, 0.01)
+    with nb.Simulation(syn.to_scenario(desc), 0.01, nb.CUDA(report_dispersal=True)) as sim:
+        g = sim.simulate(5, pause_before=60.0)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice=10, min_round_events=1 << 20,
+                        step_slice_max=1024, pause_before=60.0, report_dispersal=True, dispersal_cap=1 << 20)
+    assert same_stream(g.speciation, c.speciation)
+    a = np.sort(g.dispersal, order=("event_time", "gref"))
+    b = np.sort(c.dispersal, order=("event_time", "gref"))
+    assert len(a) == len(b) > 0
+    for f in ("gref", "prior_time", "event_time", "x", "y", "index", "tx", "ty", "tindex"):
+        assert np.array_equal(a[f], b[f]), f
+    rem, crem = np.sort(g.remaining, order="gref"), np.sort(c.remaining, order="gref")
+    for f in ("gref", "x", "y", "index", "last_event_time"):
+        assert np.array_equal(rem[f], crem[f]), f
