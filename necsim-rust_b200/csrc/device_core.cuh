@@ -346,8 +346,9 @@ __device__ __forceinline__ double poisson_next_event_time_lat(uint64_t loc_term,
 
 // rng.rs:163-167 sample_exponential of one sample: -ln(U(0,1]) / lambda,
 // with the logarithm shared bit for bit with the host (ln_dd.h)
-__device__ __forceinline__ double exp_sample(uint64_t d, double lambda) {
-    return __ddiv_rn(-necsim_ln(unit_open_closed(d)), lambda);
+__device__ __forceinline__ double exp_sample(uint64_t d, const PoissonConsts &pc) {
+    const double e = -necsim_ln(unit_open_closed(d));
+    return pc.inv_lambda != 0.0 ? __dmul_rn(e, pc.inv_lambda) : __ddiv_rn(e, pc.lambda);
 }
 
 // floor(time / delta_t) as u64 (poisson.rs:44, exp.rs:52)
@@ -369,7 +370,7 @@ __device__ __forceinline__ double exp_continue(uint64_t loc_term, double time, c
     double slice_end = __dmul_rn(__ull2double_rn(ts + 1), p.delta_t);
     for (;;) {
         j += 1;
-        et = __dadd_rn(et, exp_sample(draw_at(s0, j), pc.lambda));
+        et = __dadd_rn(et, exp_sample(draw_at(s0, j), pc));
         if (et >= slice_end) {
             ts += 1;
             j = 0;

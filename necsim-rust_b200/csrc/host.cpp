@@ -499,6 +499,11 @@ PoissonConsts make_poisson_consts(double lambda, double delta_t) {
     PoissonConsts c;
     std::memset(&c, 0, sizeof(c));
     c.lambda = lambda;
+    // x / lambda is x * (1 / lambda), exactly, for a power of two (an
+    // exponential sample is below 40)
+    int exp2 = 0;
+    const double mant = std::frexp(lambda, &exp2);
+    c.inv_lambda = mant == 0.5 && exp2 > -500 && exp2 < 500 ? 1.0 / lambda : 0.0;
     c.lambda_dt = lambda * delta_t;  // poisson.rs:40
     const double p0 = std::exp(-c.lambda_dt);  // poisson.rs:42
     for (int k = 1; k <= kPoissonTable; ++k) c.lambda_dt_over_k[k - 1] = c.lambda_dt / (double)k;

@@ -410,7 +410,7 @@ __device__ __forceinline__ double exp_search_coop(uint64_t loc_term, double time
     for (;;) {
         const uint64_t ts = base + (lane >> 3);
         const uint64_t mine = (uint64_t)(lane & 7u) + 1u;  // this lane's sample of the bucket
-        const double e = exp_sample(draw_at(primed_state(loc_term, ts), (uint32_t)mine), pc.lambda);
+        const double e = exp_sample(draw_at(primed_state(loc_term, ts), (uint32_t)mine), pc);
         const uint64_t sc = primed_state(loc_term, ts + kInvPhi * mine);
         const uint64_t c1 = draw_at(sc, 1), c2 = draw_at(sc, 2), c3 = draw_at(sc, 3), c4 = draw_at(sc, 4);
         const double slice_end = __dmul_rn(__ull2double_rn(ts + 1), p.delta_t);
@@ -1707,14 +1707,17 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
     // the SMs won the race for the queue (30,000 lineages: 26.6 warps active
     // on the busiest SM, 0.1 on the idlest).  30,000 lineages 3.5 -> 7.4e9
     // events per second, 46,000 5.4 -> 9.8e9.
-    if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * blockDim.x >= n) return;
+    // (a warp per lineage: the exponential sampler's sparse rounds, and all
+    // WrappingNoise ones)
+    const bool by_warp = EXP && (KIND == kWrappingNoise || n <= (uint64_t)gridDim.x * (blockDim.x / 32u));
+    const unsigned warps = by_warp ? warps_taking_part(a, n, blockDim.x / 32u) : 0u;
+    if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * (by_warp ? warps : blockDim.x) >= n) return;
     if (block_leaves(a.gate, a.gate_role, a.blocks_done)) return;
     const SimParams *P = stage_params<SINGLE>(a, params_smem);
     const EventSink sink = sink_of(a);
     const unsigned lane_id = threadIdx.x & 31u;
-    // (a WrappingNoise target takes a whole warp: every round)
-    if (EXP && (KIND == kWrappingNoise || n <= (uint64_t)gridDim.x * (blockDim.x / 32u))) {
-        coop_body<KIND, SINGLE, true>(a, P, n);
+    if (by_warp) {
+        if (threadIdx.x / 32u < warps) coop_body<KIND, SINGLE, true>(a, P, n);
         block_arrives(a.gate, a.gate_role, a.blocks_done);
         return;
     }
@@ -1723,6 +1726,16 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
     bool have = false;
     bool exhausted = (n == 0);
     Lane l;
+// Where a warp steps a lineage, lineages are spread over the SMs before a
+// second one joins a warp scheduler: the warps of a block that take part are
+// one per SM, then two and so on until all do, then further blocks
+// (consecutive blocks sit on different SMs).  The 64-simulation sweep's
+// rounds with 145 to 754 lineages: 75 -> 51 ms.
+__device__ __forceinline__ unsigned warps_taking_part(const StepArgs &a, uint64_t n, unsigned block_warps) {
+    if (a.gate_role != kGateNone || n >= (uint64_t)a.n_sms * block_warps) return block_warps;
+    return (unsigned)((n + a.n_sms - 1) / a.n_sms);
+}
+
     uint64_t local_steps = 0;
     uint32_t moved = 0;  // events of the lane's lineage in this launch
     Pass ps;  // converged form
@@ -1806,13 +1819,7 @@ __global__ void __launch_bounds__(kCoopBlock) coop_kernel(StepArgs a) {
     __shared__ __align__(16) unsigned char params_smem[SINGLE ? sizeof(SimParams) : 16];
     const uint64_t n = *a.n_cur;
     if (n == 0 || n > a.coop_max) return;
-    // Lineages are spread over the SMs before a second one joins a warp
-    // scheduler: one warp of a block per SM, then two, three and all four,
-    // then further blocks (consecutive blocks sit on different SMs).  The
-    // 64-simulation sweep's rounds with 145 to 754 lineages: 75 -> 51 ms.
-    const unsigned warps = a.gate_role == kGateNone && n < (uint64_t)a.n_sms * (kCoopBlock / 32)
-                               ? (unsigned)((n + a.n_sms - 1) / a.n_sms)
-                               : kCoopBlock / 32;
+    const unsigned warps = warps_taking_part(a, n, kCoopBlock / 32);
     if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * warps >= n) return;
     if (block_leaves(a.gate, a.gate_role, a.blocks_done)) return;
     const SimParams *P = stage_params<SINGLE>(a, params_smem);

@@ -85,6 +85,7 @@ struct alignas(16) PoissonConsts {
     double lambda;            // turnover rate
     double lambda_dt;         // lambda * delta_t   (poisson.rs:40)
     double lambda_dt_over_k[kPoissonTable];  // lambda_dt / k, k = 1..16
+    double inv_lambda;        // 1 / lambda when lambda is a power of two, else 0
 };
 static_assert(sizeof(PoissonConsts) % 16 == 0, "PoissonConsts must be whole 16-byte words");
 
