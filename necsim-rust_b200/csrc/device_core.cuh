@@ -504,6 +504,88 @@ __device__ __forceinline__ void normal_dispersal_draw(uint64_t d0, uint64_t d1, 
     clamp_round_dispersal(x, y, dx, dy, tx, ty);
 }
 
+// 2 pi (u - 1/2) of a sample's uniform u (2 pi 2^-32 times its high word's
+// distance from 2^31), in [-pi, pi].
+__device__ __forceinline__ float fast_angle(uint64_t d) {
+    return __fmul_rn(__int2float_rn((int)((uint32_t)(d >> 32) ^ 0x80000000u)), 0x1.921fb6p-30f);
+}
+
+// The location (dx, dy) rounded to integers away, from displacements known
+// within `margin`: false when a half is that near (or nothing is known).
+__device__ __forceinline__ bool nearest_fast(float dx, float dy, float margin, uint32_t x, uint32_t y, uint32_t &tx,
+                                             uint32_t &ty) {
+    // the nearest integer in the mantissa of v + 1.5 2^23 (|v| < 2^22; the
+    // margin of a larger displacement exceeds 1/2)
+    constexpr float kShift = 12582912.0f;
+    const float mx = __fadd_rn(dx, kShift), my = __fadd_rn(dy, kShift);
+    tx = x + (uint32_t)(__float_as_int(mx) - 0x4b400000);
+    ty = y + (uint32_t)(__float_as_int(my) - 0x4b400000);
+    const float clear = 0.5f - margin;
+    return fabsf(__fsub_rn(dx, __fsub_rn(mx, kShift))) < clear && fabsf(__fsub_rn(dy, __fsub_rn(my, kShift))) < clear;
+}
+
+// The Normal target from 32-bit arithmetic where that decides the rounding
+// (round_onto_plane only keeps the nearest integers of the displacement), a
+// lone warp's f64 logarithm, square root, sine and cosine being two thirds of
+// its event.  Returns false when the target may differ from
+// normal_dispersal_draw's, which then computes it.
+//
+// Error of dx against the real-valued displacement, for 0 <= sigma <= 64,
+// with the documented errors of the approximate functions: u0 from the high
+// word of its sample, at least 2^-10, is within 2^-21.7 of itself; __logf
+// adds 2^-21.41 on [1/2, 2], else 3 ulp (|ln u0| < 7), so r^2 = -2 ln u0 >=
+// 2^-8 is within 2^-19.5 (u0 >= 1/2: r >= 2^-4) or 2^-18 (r > 1.1) and r,
+// by sqrt.approx (2^-23), within 2^-16.4; the angle 2 pi (u1 - 1/2) in
+// [-pi, pi] is within 2^-20.8 and __sinf / __cosf add 2^-21.1.  With
+// r < 3.8 the product is within 2^-16 sigma, the f64 path within 2^-48 sigma:
+// 2^-15 sigma is kept clear of halves.  One event in about 250 is not
+// decided at sigma = 10.  Against the f64 path on 4.3e10 sample pairs (sigma
+// 0.4 to 64; Clark2Dt 1.7e10, eight shapes): no decided target differs, the
+// largest displacement error is 2^-19.1 sigma (Clark2Dt: 0.26 of its margin).
+__device__ __forceinline__ bool normal_dispersal_fast(uint64_t d0, uint64_t d1, float sigma, uint32_t x, uint32_t y,
+                                                      uint32_t &tx, uint32_t &ty) {
+    const uint32_t h0 = (uint32_t)(d0 >> 32);
+    const float r2 = -2.0f * __logf(__fmul_rn(__uint2float_rn(h0), 0x1p-32f));
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(r2));
+    // sin(-2 pi u) = sin(2 pi (u - 1/2)), cos(2 pi u) = -cos(2 pi (u - 1/2))
+    const float a = fast_angle(d1), scaled = __fmul_rn(r, sigma);
+    const bool near = nearest_fast(__fmul_rn(scaled, __sinf(a)), __fmul_rn(scaled, -__cosf(a)), 0x1p-15f * sigma, x, y,
+                                   tx, ty);
+    return h0 >= (1u << 22) && r2 >= 0x1p-8f && near;
+}
+constexpr double kFastSigma = 64.0;  // normal_dispersal_fast's largest sigma
+
+__device__ __forceinline__ void normal_target(uint64_t d0, uint64_t d1, double sigma, uint32_t x, uint32_t y,
+                                              uint32_t &tx, uint32_t &ty) {
+    if (!(sigma <= kFastSigma && normal_dispersal_fast(d0, d1, (float)sigma, x, y, tx, ty)))
+        normal_dispersal_draw(d0, d1, sigma, x, y, tx, ty);
+}
+
+// The Clark2Dt target the same way (f64: clark2dt_dispersal_draw).  With
+// y = 1 - u01 (its 53-bit integer rounded to 32 bits: 2^-24), l = log2 y and
+// w1 = 2^(-e l) = base^e, lg2.approx is within 2^-22 max(1, |l|) and
+// ex2.approx within 2^-22 of its value (PTX ISA), so w1 is within
+// eps = (e max(1, |l|) + 1) 2^-21 of itself, w = w1 - 1 within (1 + 1/w) eps,
+// the jump sqrt(u w) within (1 + 1/w) eps / 2 + 2^-22, and the displacements,
+// with __cosf and __sinf as above, within jump ((1 + 1/w) eps / 2 + 2^-19.9).
+__device__ __forceinline__ bool clark2dt_dispersal_fast(uint64_t d0, uint64_t d1, float shape_u, float exponent,
+                                                        uint32_t x, uint32_t y, uint32_t &tx, uint32_t &ty) {
+    const float yf = __fmul_rn(__ull2float_rn((1ULL << 53) - (d0 >> 11)), 0x1p-53f);
+    float l, w1, jump, inv_w;
+    asm("lg2.approx.f32 %0, %1;" : "=f"(l) : "f"(yf));
+    asm("ex2.approx.f32 %0, %1;" : "=f"(w1) : "f"(__fmul_rn(-exponent, l)));
+    const float w = __fsub_rn(w1, 1.0f);
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(jump) : "f"(__fmul_rn(shape_u, w)));
+    asm("rcp.approx.f32 %0, %1;" : "=f"(inv_w) : "f"(w));
+    const float eps = __fmul_rn(__fadd_rn(__fmul_rn(exponent, fmaxf(1.0f, -l)), 1.0f), 0x1p-21f);
+    const float margin =
+        __fmul_rn(jump, __fadd_rn(__fmul_rn(__fadd_rn(1.0f, inv_w), __fmul_rn(eps, 0.75f)), 0x1p-19f));
+    const float a = fast_angle(d1);  // cos(2 pi u) = -cos(a), sin(2 pi u) = -sin(a)
+    const bool near = nearest_fast(__fmul_rn(jump, -__cosf(a)), __fmul_rn(jump, -__sinf(a)), margin, x, y, tx, ty);
+    return w >= 0x1p-12f && near;
+}
+
 // landscape/extent.rs:44-49 LandscapeExtent::contains for the SI local
 // extent, whose origin is (0, 0)
 __device__ __forceinline__ bool in_local(const SimParams &p, uint32_t x, uint32_t y) {

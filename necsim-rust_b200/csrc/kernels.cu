@@ -255,10 +255,13 @@ __device__ __forceinline__ bool event_target(const Lane &l, const SimParams &p, 
         ti = coalescence_index(d_coal, in_local(p, tx, ty) ? p.deme : p.meta_deme);
     } else if (KIND == kAlmostInfiniteNormal) {
         // sample e4 is CoalescenceRngSample::new's draw; singleton demes -> index 0
-        if (p.clark)
-            clark2dt_dispersal_draw(e2, e3, p.clark_shape_u, p.clark_exponent, l.x, l.y, tx, ty);
-        else
-            normal_dispersal_draw(e2, e3, p.sigma, l.x, l.y, tx, ty);
+        // (in 32-bit arithmetic where that decides the rounding)
+        if (p.clark) {
+            if (!clark2dt_dispersal_fast(e2, e3, (float)p.clark_shape_u, (float)p.clark_exponent, l.x, l.y, tx, ty))
+                clark2dt_dispersal_draw(e2, e3, p.clark_shape_u, p.clark_exponent, l.x, l.y, tx, ty);
+        } else {
+            normal_target(e2, e3, p.sigma, l.x, l.y, tx, ty);
+        }
         ti = 0;
     } else if (KIND == kWrappingNoise) {
         // dispersal_sampler/wrapping_noise.rs:42-87: self-dispersal iff
@@ -270,7 +273,7 @@ __device__ __forceinline__ bool event_target(const Lane &l, const SimParams &p, 
         if ((e2 >> 11) >= p.noise.self_threshold) {
             uint64_t d0 = e3, d1 = EAGER ? e4 : draw_at(rs, 4);
             for (uint32_t c = 0;; ++c) {
-                normal_dispersal_draw(d0, d1, p.sigma, l.x, l.y, tx, ty);
+                normal_target(d0, d1, p.sigma, l.x, l.y, tx, ty);
                 if ((tx != l.x || ty != l.y) && noise::habitat_at(p.noise, tx, ty) != 0) break;
                 if (c + 1 == kMaxDispersalRejections) {
                     err |= kErrDispersalRejections;
@@ -534,7 +537,7 @@ __device__ __forceinline__ bool noise_target_coop(const SimParams &p, const Nois
         const int src = 2 * (int)(lane & (kTargets - 1u));
         const uint64_t d0 = __shfl_sync(kFull, d, src), d1 = __shfl_sync(kFull, d, src + 1);
         uint32_t cx, cy;
-        normal_dispersal_draw(d0, d1, p.sigma, x, y, cx, cy);
+        normal_target(d0, d1, p.sigma, x, y, cx, cy);
         unsigned open = __ballot_sync(kFull, lane < kTargets && (cx != x || cy != y));
         int found = -1;
         if (h.coverage >= 1.0) {
@@ -962,11 +965,11 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
 //    with the event computed.
 // Measured with one lineage on a B200 (1,965 MHz), coop_run -> chain_run:
 // NonSpatial 1,772 -> 673 cycles per event, SpatiallyImplicit 1,747 -> 663,
-// AlmostInfinite Normal 2,793 -> 1,503, Clark2Dt 3,376 -> 2,173 (1,892 and
-// 2,568 with separate sin and cos), SpatiallyExplicit 3,019 -> 2,341 (64 x 64
+// AlmostInfinite Normal 2,793 -> 731, Clark2Dt 3,376 -> 725 (1,503 and 2,173
+// with f64 displacements), SpatiallyExplicit 3,019 -> 2,341 (64 x 64
 // map; its atoms, 190 MB, come from HBM).  The bound is the instruction count: a
 // lone warp issues one instruction every two cycles, and NonSpatial takes 329
-// per event (48 a prime, 31 a sample), AlmostInfinite Normal 524.
+// per event (48 a prime, 31 a sample).
 template <int KIND>
 constexpr bool kChainKind = KIND != kWrappingNoise;
 
@@ -1065,7 +1068,11 @@ struct Chain {
 // Events of a lineage in one community (LOCAL: SpatiallyImplicit's local
 // one, which it leaves by migration: kStepMoved) until it stops
 // (kStepStop, with the peek) or speciates (kStepSpeciated, at c.next).
-template <int KIND, bool LOCAL>
+// FAST: AlmostInfinite targets in 32-bit arithmetic where that decides them
+// (kFastNormal and kFastClark are loops of their own: together, one lineage
+// took 804 and 888 cycles per event).
+constexpr int kFastNone = 0, kFastNormal = 1, kFastClark = 2;
+template <int KIND, bool LOCAL, int FAST = kFastNone>
 __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p, const EventSink &k,
                                            const volatile unsigned *stop) {
     constexpr bool kMigrates = KIND == kSpatiallyImplicit && LOCAL;
@@ -1109,6 +1116,7 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
     const double deme_u = __dmul_rn(__uint2double_rn(com.deme), 0x1p-53);
     const uint64_t deme_k = (uint64_t)com.deme * kSeaHashK;
     const double sigma = p.sigma, horizon = __dmul_rn(l.horizon, p.inv_delta_t);
+    const float sigma_f = (float)sigma, shape_f = (float)p.clark_shape_u, exponent_f = (float)p.clark_exponent;
     const bool clark = p.clark != 0;
 
     constexpr uint32_t kFlush = 1u << 30;  // `moved` is added up before it overflows
@@ -1142,10 +1150,12 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
             leave = (kMigrates ? d2 : d1) <= leave_at_most;
             uint64_t inj_k;
             if constexpr (KIND == kAlmostInfiniteNormal) {
-                if (clark)
-                    clark2dt_dispersal_draw(d2, d3, p.clark_shape_u, p.clark_exponent, c.x, c.y, tx, ty);
+                if (FAST == kFastNormal)
+                    leave = !normal_dispersal_fast(d2, d3, sigma_f, c.x, c.y, tx, ty) || leave;
+                else if (FAST == kFastClark)
+                    leave = !clark2dt_dispersal_fast(d2, d3, shape_f, exponent_f, c.x, c.y, tx, ty) || leave;
                 else
-                    normal_dispersal_draw(d2, d3, sigma, c.x, c.y, tx, ty);
+                    normal_dispersal_draw(d2, d3, sigma, c.x, c.y, tx, ty);  // (Clark2Dt is always fast)
                 inj_k = (((uint64_t)ty << 32) | (uint64_t)tx) * kSeaHashK;
             } else if constexpr (KIND == kSpatiallyExplicit) {
                 // packed_separable_alias/dispersal.rs:16-77 (the cases of
@@ -1298,9 +1308,21 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
             if (lane == 0) set_status(k.status, bits);
             return kStepDropped;
         }
-        if (leaves && !kMigrates) return kStepSpeciated;
+        // (FAST: or the target is not decided)
+        if (leaves && !kMigrates && (!FAST || __shfl_sync(kFull, d1 <= leave_at_most ? 1 : 0, (int)cand)))
+            return kStepSpeciated;
         if (k.report_dispersal && lane == 0) chain_unpack<KIND>(p, c.loc_term, LOCAL, c.cell, l.x, l.y, l.i);
-        if (leaves) {
+        if (FAST && leaves) {
+            const uint64_t s_e = __shfl_sync(kFull, s, (int)cand);
+            const uint64_t d2 = draw_at(s_e, 2), d3 = draw_at(s_e, 3);
+            if (clark)
+                clark2dt_dispersal_draw(d2, d3, p.clark_shape_u, p.clark_exponent, c.x, c.y, tx, ty);
+            else
+                normal_dispersal_draw(d2, d3, sigma, c.x, c.y, tx, ty);
+            c.x = tx;
+            c.y = ty;
+            c.loc_term = location_term(p.seed, ((uint64_t)ty << 32) | (uint64_t)tx);
+        } else if (leaves) {
             // migration: the target in the metacommunity from samples 3 and 4
             const uint64_t s_e = __shfl_sync(kFull, s, (int)cand);
             const Community meta = community_of<KIND>(p, false);
@@ -1329,7 +1351,7 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
         c.before = c.next;
         c.base = f64_to_u64(floor(c.next));
         c.moved += 1;
-        if (leaves) return kStepMoved;
+        if (kMigrates && leaves) return kStepMoved;
         if (c.moved >= kFlush) {
             l.steps += c.moved;
             c.moved = 0;
@@ -1363,7 +1385,13 @@ __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const Even
         result = chain_phase<KIND, true>(c, l, p, k, stop);
         c.local = result != kStepMoved;
     }
-    if (result == kStepMoved) result = chain_phase<KIND, KIND != kSpatiallyImplicit>(c, l, p, k, stop);
+    constexpr bool kPlane = KIND == kAlmostInfiniteNormal;
+    if (kPlane && p.clark)
+        result = chain_phase<KIND, true, kPlane ? kFastClark : kFastNone>(c, l, p, k, stop);
+    else if (kPlane && p.sigma <= kFastSigma)
+        result = chain_phase<KIND, true, kPlane ? kFastNormal : kFastNone>(c, l, p, k, stop);
+    else if (result == kStepMoved)
+        result = chain_phase<KIND, KIND != kSpatiallyImplicit>(c, l, p, k, stop);
     l.steps += c.moved;
     if (l.steps != steps) l.last = __dmul_rn(c.before, p.delta_t);
     if (result == kStepSpeciated) l.steps += 1;
@@ -1695,6 +1723,16 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
     if (a.steps_total && lane_id == 0 && warp_steps) atomicAdd(a.steps_total, (unsigned long long)warp_steps);
 }
 
+// Where a warp steps a lineage, lineages are spread over the SMs before a
+// second one joins a warp scheduler: the warps of a block that take part are
+// one per SM, then two and so on until all do, then further blocks
+// (consecutive blocks sit on different SMs).  The 64-simulation sweep's
+// rounds with 145 to 754 lineages: 75 -> 51 ms.
+__device__ __forceinline__ unsigned warps_taking_part(const StepArgs &a, uint64_t n, unsigned block_warps) {
+    if (a.gate_role != kGateNone || n >= (uint64_t)a.n_sms * block_warps) return block_warps;
+    return (unsigned)((n + a.n_sms - 1) / a.n_sms);
+}
+
 template <int KIND, bool SINGLE, bool EXP>
 __device__ __forceinline__ void step_body(const StepArgs &a) {
     // one simulation: its parameters live in shared memory for the launch
@@ -1726,16 +1764,6 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
     bool have = false;
     bool exhausted = (n == 0);
     Lane l;
-// Where a warp steps a lineage, lineages are spread over the SMs before a
-// second one joins a warp scheduler: the warps of a block that take part are
-// one per SM, then two and so on until all do, then further blocks
-// (consecutive blocks sit on different SMs).  The 64-simulation sweep's
-// rounds with 145 to 754 lineages: 75 -> 51 ms.
-__device__ __forceinline__ unsigned warps_taking_part(const StepArgs &a, uint64_t n, unsigned block_warps) {
-    if (a.gate_role != kGateNone || n >= (uint64_t)a.n_sms * block_warps) return block_warps;
-    return (unsigned)((n + a.n_sms - 1) / a.n_sms);
-}
-
     uint64_t local_steps = 0;
     uint32_t moved = 0;  // events of the lane's lineage in this launch
     Pass ps;  // converged form

@@ -50,6 +50,10 @@ CASES = {
     "wide_displacements": (ai(4, 3e8, 0.01), {}, None),
     "no_displacement": (ai(4, 0.0, 0.01, centre=(1, M32)), {}, None),
     "narrow_displacements": (ai(5, 0.4, 0.01, centre=(1, M32)), {}, None),
+    "sigma_64": (ai(5, 64.0, 0.002), {}, None),  # the widest that 32-bit arithmetic decides
+    "sigma_above_64": (ai(5, 64.0001, 0.002), {}, None),
+    "clark_tiny": (dict(kind=4, speciation_probability=0.005, shape_u=1e-9, tail_p=3.0, radius=4, centre_x=2,
+                        centre_y=M32 - 1), {}, None),
     "clark_wide": (dict(kind=4, speciation_probability=0.01, shape_u=1e9, tail_p=1.0, radius=4, centre_x=2,
                         centre_y=M32 - 1), {}, None),
 }
@@ -194,3 +198,19 @@ def test_explicit_dispersal_events(nb, syn, oracle):
     rem, crem = np.sort(g.remaining, order="gref"), np.sort(c.remaining, order="gref")
     for f in ("gref", "x", "y", "index", "last_event_time"):
         assert np.array_equal(rem[f], crem[f]), f
+
+
+@pytest.mark.parametrize("desc", [
+    dict(kind=2, sigma=10.0), dict(kind=2, sigma=0.7), dict(kind=2, sigma=60.0),
+    dict(kind=4, shape_u=4.0, tail_p=0.5), dict(kind=4, shape_u=1.0, tail_p=1.0), dict(kind=4, shape_u=20.0, tail_p=0.4),
+], ids=lambda d: "-".join("%s" % v for v in d.values()))
+def test_displacements_decided_in_32_bits(nb, syn, oracle, desc):
+    """Some 10^6 events: several thousand targets are not decided by the 32-bit
+    arithmetic; one wrong rounding would move a lineage for good.  (The steep
+    Clark2Dt tails reach beyond 2^32 cells.)"""
+    desc = dict(desc, speciation_probability=1e-3, radius=18, centre_x=M32 // 2, centre_y=3)
+    g = nb.simulate(1e-3, syn.to_scenario(desc), 9)
+    c = oracle.simulate(desc, 9, mode=oracle.MODE_CANONICAL, step_slice=10, min_round_events=1 << 20,
+                        step_slice_max=1024)
+    assert g.steps == c.steps > 500_000
+    assert same_stream(g.speciation, c.speciation)
