@@ -28,31 +28,10 @@ constexpr uint64_t kInvPhi = 0x9e3779b97f4a7c15ULL;
 // core::f64::consts::TAU
 constexpr double kTau = 6.283185307179586;
 
-// The 128-bit product of two 64-bit words from four 32 x 32 -> 64 products
-// (separate low and high product instructions would take seven).
-__device__ __forceinline__ uint64_t mul_wide(uint32_t a, uint32_t b) { return (uint64_t)a * (uint64_t)b; }
-__device__ __forceinline__ void mul_64_64(uint64_t a, uint64_t b, uint64_t &lo, uint64_t &hi) {
-    const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
-    const uint64_t p00 = mul_wide(a0, b0), p01 = mul_wide(a0, b1), p10 = mul_wide(a1, b0), p11 = mul_wide(a1, b1);
-    uint32_t l1, h0, h1;
-    asm("{\n\t.reg .u32 t1, t2, t3;\n\t"
-        "add.cc.u32 t1, %3, %4;\n\t"
-        "addc.cc.u32 t2, %5, %6;\n\t"
-        "addc.u32 t3, %7, 0;\n\t"
-        "add.cc.u32 %0, t1, %8;\n\t"
-        "addc.cc.u32 %1, t2, %9;\n\t"
-        "addc.u32 %2, t3, 0;\n\t}"
-        : "=r"(l1), "=r"(h0), "=r"(h1)
-        : "r"((uint32_t)(p00 >> 32)), "r"((uint32_t)p01), "r"((uint32_t)(p01 >> 32)), "r"((uint32_t)p11),
-          "r"((uint32_t)(p11 >> 32)), "r"((uint32_t)p10), "r"((uint32_t)(p10 >> 32)));
-    lo = ((uint64_t)l1 << 32) | (uint32_t)p00;
-    hi = ((uint64_t)h1 << 32) | h0;
-}
-
 // wyhash.rs:85-96: 64x64 -> 128 multiply, low and high halves xor-folded
 __device__ __forceinline__ uint64_t wymum(uint64_t a, uint64_t b) {
-    uint64_t lo, hi;
-    mul_64_64(a, b, lo, hi);
+    const uint64_t lo = a * b;
+    const uint64_t hi = __umul64hi(a, b);
     return (a ^ lo) ^ (b ^ hi);
 }
 
@@ -143,9 +122,8 @@ __device__ __forceinline__ uint64_t primed_state(uint64_t loc_term, uint64_t tim
 // the k-th sample_u64 after priming to s0
 __device__ __forceinline__ uint64_t draw_at(uint64_t s0, uint32_t k) {
     const uint64_t s = s0 + (uint64_t)k * kWyP0;
-    uint64_t lo, hi;
-    mul_64_64(s ^ kWyP1, s, lo, hi);
-    return seahash_diffuse(lo ^ hi ^ kWyP1);  // wymum(s ^ P1, s): its factors' xor is P1
+    const uint64_t a = s ^ kWyP1, lo = a * s, hi = __umul64hi(a, s);
+    return seahash_diffuse(lo ^ hi ^ kWyP1);  // wymum(a, s): the factors' xor is P1
 }
 
 __device__ __forceinline__ double unit_closed_open(uint64_t v) {
