@@ -528,8 +528,7 @@ PoissonConsts make_poisson_consts(double lambda, double delta_t) {
 // where it reaches into the local extent, the reference tests local first).
 bool chain_scenario(const SimParams &p, int32_t kind) {
     const uint64_t most = 0xffffffffULL;
-    // a power of two whose products with event times stay normal
-    if (p.inv_delta_t == 0.0 || !(p.delta_t > 0x1p-256 && p.delta_t < 0x1p256)) return false;
+    if (!(p.delta_t > 0x1p-256 && p.delta_t < 0x1p256)) return false;  // products with event times stay normal
     switch (kind) {
     case NECSIM_NON_SPATIAL: return (uint64_t)p.width * p.height <= most;
     case NECSIM_SPATIALLY_IMPLICIT:
@@ -595,7 +594,8 @@ SimParams base_params(const necsim_scenario &sc, const necsim_args &args, uint64
         p.clark_exponent = 1.0 / sc.tail_p;
     }
     if (sc.kind == NECSIM_WRAPPING_NOISE) p.noise = noise_habitat(sc);
-    p.chain = chain_scenario(p, sc.kind) ? 1 : 0;
+    // (the Poisson form works in units of delta_t, a power of two)
+    if (chain_scenario(p, sc.kind)) p.chain = kChainExp | (p.inv_delta_t != 0.0 ? kChainPoisson : 0);
     p.pause_before = -1.0;
     return p;
 }

@@ -973,13 +973,13 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
 template <int KIND>
 constexpr bool kChainKind = KIND != kWrappingNoise;
 
-// Whether chain_run takes the simulation's round: SimParams.chain (delta_t a
-// power of two, every table length below 2^32, no metacommunity cell inside
+// Whether chain_run takes the simulation's round: SimParams.chain (for the
+// Poisson sampler delta_t a power of two, every table length below 2^32, no metacommunity cell inside
 // the local community) and time buckets that are exact doubles.
-template <int KIND>
+template <int KIND, bool EXP>
 __device__ __forceinline__ bool chain_takes(const SimParams &p, const Lane &l) {
     const double most = __dmul_rn(p.delta_t, 0x1p50);
-    return kChainKind<KIND> && p.chain != 0 && l.horizon < most && l.last < most && p.min_event_time < most;
+    return kChainKind<KIND> && (p.chain & (EXP ? kChainExp : kChainPoisson)) != 0 && l.horizon < most && l.last < most && p.min_event_time < most;
 }
 
 // A bucket lane's search result, one word that orders by bucket: buckets
@@ -1055,8 +1055,9 @@ struct Chain {
     uint64_t loc_term;
     uint64_t base;       // time bucket the search starts in
     uint64_t reprime;    // of a peeked event
-    double before;       // the search's start, in units of delta_t
-    double next;         // peeked event time, in units of delta_t
+    // in units of delta_t (exponential sampler: of time)
+    double before;       // the search's start
+    double next;         // peeked event time
     uint32_t x, y;       // AlmostInfinite
     uint32_t cell;       // SpatiallyExplicit: the cell, in range, and
     CellRecord rec;      // its record
@@ -1071,21 +1072,29 @@ struct Chain {
 // FAST: AlmostInfinite targets in 32-bit arithmetic where that decides them
 // (kFastNormal and kFastClark are loops of their own: together, one lineage
 // took 804 and 888 cycles per event).
+// EXP: the exponential sampler (exp.rs:37-83).  Lane (b, j) holds sample j of
+// bucket base + b, b < 4, and the event that it would be; every lane adds up
+// its bucket's samples in order (the reference's rounding) from the others'.
+// Times are not scaled: any delta_t.
 constexpr int kFastNone = 0, kFastNormal = 1, kFastClark = 2;
-template <int KIND, bool LOCAL, int FAST = kFastNone>
+template <int KIND, bool LOCAL, bool EXP, int FAST = kFastNone>
 __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p, const EventSink &k,
                                            const volatile unsigned *stop) {
     constexpr bool kMigrates = KIND == kSpatiallyImplicit && LOCAL;
     const unsigned lane = threadIdx.x & 31u;
-    const bool bucket_lane = lane < kCoopBuckets;
+    const bool bucket_lane = !EXP && lane < kCoopBuckets;
     uint32_t my_b = lane, my_k = 0;
-    if (!bucket_lane) {
+    if (EXP) {
+        my_b = lane >> 3;
+        my_k = lane & 7u;
+    } else if (!bucket_lane) {
         const unsigned j = lane - kCoopBuckets;
         const uint64_t w = j < 8u ? kCoopPairWord0 : (j < 16u ? kCoopPairWord1 : kCoopPairWord2);
         const uint32_t pr = (uint32_t)(w >> (8u * (j & 7u))) & 0xffu;
         my_b = pr & 15u;
         my_k = pr >> 4;
     }
+    const uint64_t my_sample = (uint64_t)(my_k + 1u) * kWyP0;  // EXP: the search's sample
     const uint64_t my_tadd_k = ((uint64_t)my_b + (bucket_lane ? 0ULL : kInvPhi * (uint64_t)(my_k + 1u))) * kSeaHashK;
     // the keys of this bucket's events 0..2 (no candidate lane finds one)
     const uint32_t lanes_b = coop_lane_table(my_b & 7u);
@@ -1115,17 +1124,19 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
     const double cells_u = __dmul_rn(__ull2double_rn(com.cells), 0x1p-53);
     const double deme_u = __dmul_rn(__uint2double_rn(com.deme), 0x1p-53);
     const uint64_t deme_k = (uint64_t)com.deme * kSeaHashK;
-    const double sigma = p.sigma, horizon = __dmul_rn(l.horizon, p.inv_delta_t);
+    const double sigma = p.sigma, delta_t = p.delta_t;
+    const double horizon = EXP ? l.horizon : __dmul_rn(l.horizon, p.inv_delta_t);
     const float sigma_f = (float)sigma, shape_f = (float)p.clark_shape_u, exponent_f = (float)p.clark_exponent;
     const bool clark = p.clark != 0;
 
     constexpr uint32_t kFlush = 1u << 30;  // `moved` is added up before it overflows
-    uint64_t tk = 0, start_bits = 0;
+    uint64_t tk = 0, search_k = 0, start_bits = 0;
     // the event count at which the inner loop is left: to look at `stop`, for
     // a peeked event, and at every event when dispersal events are reported
     uint32_t attend = 0;
     auto enter = [&] {
         tk = c.peek ? c.reprime * kSeaHashK : c.base * kSeaHashK + my_tadd_k;
+        search_k = (c.base + my_b) * kSeaHashK;  // EXP
         start_bits = 0x4330000000000000ULL | (c.base + my_b);
         attend = c.peek || k.report_dispersal ? c.moved : (stop ? (c.moved + 31u) & ~31u : kFlush);
     };
@@ -1140,8 +1151,9 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
             // a peeked event is computed by every lane, a search by the lanes' roles
             s = primed_state_k(c.loc_term, tk);
             d1 = draw_at(s, 1);
-            const uint64_t d2 = draw_at(s, 2), d3 = draw_at(s, 3), d4 = draw_at(s, 4);
-            const double v2 = sample_bits(d2), v3 = sample_bits(d3), v4 = sample_bits(d4);
+            constexpr bool kFour = !EXP || kMigrates || KIND == kSpatiallyExplicit;
+            const uint64_t d2 = draw_at(s, 2), d3 = draw_at(s, 3), d4 = kFour ? draw_at(s, 4) : 0;
+            const double v2 = sample_bits(d2), v3 = sample_bits(d3), v4 = kFour ? sample_bits(d4) : 0.0;
 
             // candidate view: the event that this lane's samples make
             // (event_sampler/independent.rs:112-222); a local lineage never
@@ -1198,29 +1210,60 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
             loc_next = swap_halves(seahash_finish(inj_k)) ^ seed_term;
             const uint32_t next_hi = leave ? kAttention : (uint32_t)(loc_next >> 32);
 
-            // bucket view: the earliest event of this lane's bucket after
-            // `before` among its first three (ties: lowest index),
-            // poisson.rs:48-100
-            const double start = __dsub_rn(__longlong_as_double((long long)start_bits), 0x1p52);
-            const double q0 = __fma_rn(v2, 0x1p-53, start);  // start + u: u is exact
-            const double q1 = __fma_rn(v3, 0x1p-53, start);
-            const double q2 = __fma_rn(v4, 0x1p-53, start);
-            mine = d1 > more0 && q0 > c.before ? q0 : kNeverTime;
-            uint32_t key = key0;
-            if (d1 > more1 && q1 > c.before && q1 < mine) {
-                mine = q1;
-                key = key1;
+            if constexpr (EXP) {
+                // this lane's sample, and the running sum up to it
+                const double e =
+                    exp_sample(draw_at(primed_state_k(c.loc_term, search_k) + my_sample, 0), *pc);
+                const double bucket = __dsub_rn(__longlong_as_double((long long)start_bits), 0x1p52);
+                const double slice_end = __dmul_rn(__dadd_rn(bucket, 1.0), delta_t);
+                double before_mine = c.before;  // the sum before this lane's sample (the first: nothing passed)
+                const double slice_start = __dmul_rn(bucket, delta_t);
+                mine = slice_start;
+#pragma unroll
+                for (unsigned i = 0; i < 8u; ++i) {
+                    const double next_sum = __dadd_rn(mine, __shfl_sync(kFull, e, (int)((lane & 24u) + i)));
+                    if (i <= my_k) {
+                        before_mine = i ? mine : c.before;
+                        mine = next_sum;
+                    }
+                }
+                const bool inside = mine < slice_end;
+                // the first sum past `before`; or none of the eight samples is
+                // past it nor past the bucket's end: more of them decide
+                const bool hit = inside && mine > c.before && !(before_mine > c.before);
+                const bool more = inside && my_k == 7u && !(mine > c.before);
+                uint32_t key = (my_b << 28) | (lane << 20) | (my_k << 8) | lane;
+                if (mine >= horizon) key |= kSelStop;
+                // near the bucket's ends t / delta_t may round into the next or
+                // the previous one: the slow way
+                const double close = __dmul_rn(slice_end, 0x1p-50);
+                if (more || __dsub_rn(slice_end, mine) < close || __dsub_rn(mine, slice_start) < close) key |= kSelMore;
+                sel = __reduce_min_sync(kFull, hit || more ? key : kSelNone);
+            } else {
+                // bucket view: the earliest event of this lane's bucket after
+                // `before` among its first three (ties: lowest index),
+                // poisson.rs:48-100
+                const double start = __dsub_rn(__longlong_as_double((long long)start_bits), 0x1p52);
+                const double q0 = __fma_rn(v2, 0x1p-53, start);  // start + u: u is exact
+                const double q1 = __fma_rn(v3, 0x1p-53, start);
+                const double q2 = __fma_rn(v4, 0x1p-53, start);
+                mine = d1 > more0 && q0 > c.before ? q0 : kNeverTime;
+                uint32_t key = key0;
+                if (d1 > more1 && q1 > c.before && q1 < mine) {
+                    mine = q1;
+                    key = key1;
+                }
+                if (d1 > more2 && q2 > c.before && q2 < mine) {
+                    mine = q2;
+                    key = key2;
+                }
+                if (mine >= __dadd_rn(start, 1.0)) key += 1u << 28;  // rounded up (or none)
+                if (mine >= horizon) key |= kSelStop;
+                const bool more = d1 > more3;
+                if (more) key |= kSelMore;
+                const bool found = bucket_lane && (more || mine < kNeverTime);
+                sel = __reduce_min_sync(kFull, found ? key : kSelNone);
             }
-            if (d1 > more2 && q2 > c.before && q2 < mine) {
-                mine = q2;
-                key = key2;
-            }
-            if (mine >= __dadd_rn(start, 1.0)) key += 1u << 28;  // rounded up (or none)
-            if (mine >= horizon) key |= kSelStop;
-            const bool more = d1 > more3;
-            if (more) key |= kSelMore;
-            const bool found = bucket_lane && (more || mine < kNeverTime);
-            sel = __reduce_min_sync(kFull, found ? key : kSelNone);
 
             const double q = __shfl_sync(kFull, mine, (int)(sel >> 20));
             const uint32_t lo = __shfl_sync(kFull, (uint32_t)loc_next, (int)sel);
@@ -1237,6 +1280,7 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
             }
             c.loc_term = ((uint64_t)hi << 32) | lo;
             tk += (uint64_t)(sel >> 28) * kSeaHashK;
+            if (EXP) search_k += (uint64_t)(sel >> 28) * kSeaHashK;
             start_bits += sel >> 28;
             c.before = q;
             c.moved += 1;
@@ -1246,16 +1290,23 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
         uint32_t cand = lane;
         if (searched) {
             c.base = (start_bits & 0xfffffffffffffULL) - my_b;
-            if (sel == kSelNone) {  // eight empty buckets: the next eight
-                c.base += kCoopBuckets;
+            if (sel == kSelNone) {  // no event in the buckets searched: the next ones
+                c.base += EXP ? 4u : kCoopBuckets;
                 enter();
                 continue;
             }
-            const uint32_t b_sel = (sel >> 20) & 31u;
+            const uint32_t lane_sel = (sel >> 20) & 31u, b_sel = EXP ? sel >> 28 : lane_sel;
             uint32_t k_sel = (sel >> 8) & 0xffu;
             cand = sel & 0xffu;
-            double q = __shfl_sync(kFull, mine, (int)b_sel);
-            if (sel & kSelMore) {
+            double q = __shfl_sync(kFull, mine, (int)lane_sel);
+            c.reprime = c.base + b_sel + kInvPhi * (uint64_t)(k_sel + 1u);
+            if (EXP) {
+                // eight samples that decide nothing: one after the other
+                if (!(q > c.before)) {
+                    q = exp_continue(c.loc_term, c.before, p, *pc, c.base + b_sel, 8u, q, c.reprime);
+                    cand = kNoCandidate;
+                }
+            } else if (sel & kSelMore) {
                 // the bucket has more than three events (3% of the buckets
                 // with events at lambda delta_t = 1): lane j draws j, j + 32, ...
                 const uint64_t s_b = __shfl_sync(kFull, s, (int)b_sel), d1_b = __shfl_sync(kFull, d1, (int)b_sel);
@@ -1282,9 +1333,9 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
                 q = __hiloint2double((int)hi, (int)lo);
                 const uint32_t lanes_sel = __shfl_sync(kFull, lanes_b, (int)b_sel);
                 cand = k_sel < 4u ? (lanes_sel >> (8u * k_sel)) & 0xffu : kNoCandidate;
+                c.reprime = c.base + b_sel + kInvPhi * (uint64_t)(k_sel + 1u);
             }
             c.next = q;
-            c.reprime = c.base + b_sel + kInvPhi * (uint64_t)(k_sel + 1u);
             // the reference's early stop `next_event_time >= level_time`
             // (monolithic/mod.rs:228-239), or an interruption
             bool keep = q >= horizon;
@@ -1344,12 +1395,12 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
         if (k.report_dispersal && lane == 0) {
             uint32_t ex, ey, ei;
             chain_unpack<KIND>(p, c.loc_term, LOCAL && !leaves, c.cell, ex, ey, ei);
-            l.next = __dmul_rn(c.next, p.delta_t);
+            l.next = EXP ? c.next : __dmul_rn(c.next, delta_t);
             emit_dispersal(l, k, ex, ey, ei);
             l.last = l.next;
         }
         c.before = c.next;
-        c.base = f64_to_u64(floor(c.next));
+        c.base = EXP ? time_bucket(p, c.next) : f64_to_u64(floor(c.next));
         c.moved += 1;
         if (kMigrates && leaves) return kStepMoved;
         if (c.moved >= kFlush) {
@@ -1360,15 +1411,15 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
     }
 }
 
-template <int KIND>
+template <int KIND, bool EXP>
 __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const EventSink &k, uint64_t &events,
                                          const volatile unsigned *stop = nullptr) {
     Chain c;
     c.loc_term = location_term(p.seed, lane_injection<KIND>(l, p));
     const double before = l.last > p.min_event_time ? l.last : p.min_event_time;
     c.base = time_bucket(p, before);
-    c.before = __dmul_rn(before, p.inv_delta_t);
-    c.next = __dmul_rn(l.next, p.inv_delta_t);
+    c.before = EXP ? before : __dmul_rn(before, p.inv_delta_t);
+    c.next = EXP ? l.next : __dmul_rn(l.next, p.inv_delta_t);
     c.reprime = l.reprime;
     c.peek = l.has_next;
     c.x = l.x;
@@ -1382,21 +1433,21 @@ __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const Even
     const uint64_t steps = l.steps;
     int result = kStepMoved;
     if (KIND == kSpatiallyImplicit && c.local) {
-        result = chain_phase<KIND, true>(c, l, p, k, stop);
+        result = chain_phase<KIND, true, EXP>(c, l, p, k, stop);
         c.local = result != kStepMoved;
     }
     constexpr bool kPlane = KIND == kAlmostInfiniteNormal;
     if (kPlane && p.clark)
-        result = chain_phase<KIND, true, kPlane ? kFastClark : kFastNone>(c, l, p, k, stop);
+        result = chain_phase<KIND, true, EXP, kPlane ? kFastClark : kFastNone>(c, l, p, k, stop);
     else if (kPlane && p.sigma <= kFastSigma)
-        result = chain_phase<KIND, true, kPlane ? kFastNormal : kFastNone>(c, l, p, k, stop);
+        result = chain_phase<KIND, true, EXP, kPlane ? kFastNormal : kFastNone>(c, l, p, k, stop);
     else if (result == kStepMoved)
-        result = chain_phase<KIND, KIND != kSpatiallyImplicit>(c, l, p, k, stop);
+        result = chain_phase<KIND, KIND != kSpatiallyImplicit, EXP>(c, l, p, k, stop);
     l.steps += c.moved;
-    if (l.steps != steps) l.last = __dmul_rn(c.before, p.delta_t);
+    if (l.steps != steps) l.last = EXP ? c.before : __dmul_rn(c.before, p.delta_t);
     if (result == kStepSpeciated) l.steps += 1;
     events += l.steps - steps;
-    l.next = __dmul_rn(c.next, p.delta_t);
+    l.next = EXP ? c.next : __dmul_rn(c.next, p.delta_t);
     l.reprime = c.reprime;
     l.has_next = result == kStepStop;
     chain_unpack<KIND>(p, c.loc_term, c.local, c.cell, l.x, l.y, l.i);
@@ -1410,7 +1461,7 @@ template <int KIND>
 __device__ __forceinline__ int warp_run(Lane &l, const SimParams &p, const EventSink &k, uint64_t &events,
                                         const volatile unsigned *stop = nullptr) {
     if constexpr (kChainKind<KIND>) {
-        if (chain_takes<KIND>(p, l)) return chain_run<KIND>(l, p, k, events, stop);
+        if (chain_takes<KIND, false>(p, l)) return chain_run<KIND, false>(l, p, k, events, stop);
     }
     return coop_run<KIND>(l, p, k, events, stop);
 }
@@ -1646,7 +1697,11 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
         int r;
         if constexpr (EXP) {
             uint32_t moved = 0;
-            for (;;) {
+            const bool chain = chain_takes<KIND, true>(p, c);
+            if constexpr (kChainKind<KIND>) {
+                if (chain) r = chain_run<KIND, true>(c, p, sink, warp_steps);
+            }
+            while (!chain) {
                 r = lineage_step_coop<KIND, true>(c, p, sink, noise_lanes);
                 if (r != kStepMoved) break;
                 warp_steps += 1;
@@ -1655,7 +1710,7 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
                     break;
                 }
             }
-            if (r == kStepSpeciated) warp_steps += 1;
+            if (!chain && r == kStepSpeciated) warp_steps += 1;
         } else {
             if constexpr (!kChainKind<KIND>) {
                 // the speculative candidates' alias and record reads cost more
@@ -1964,7 +2019,13 @@ __global__ void __launch_bounds__(THREADS, 1) resident_kernel(ResidentArgs a) {
                     bool c_live = true;
                     if constexpr (EXP || KIND == kWrappingNoise) {
                         const NoiseLane noise_lanes = noise_lane<KIND>(p);
-                        for (;;) {
+                        const bool chain = EXP && chain_takes<KIND, true>(p, c);
+                        if constexpr (EXP && kChainKind<KIND>) {
+                            uint64_t ev = 0;
+                            if (chain) c_live = chain_run<KIND, true>(c, p, sink, ev) == kStepStop;
+                            my_events += ev;
+                        }
+                        while (!chain) {
                             const int r = lineage_step_coop<KIND, EXP>(c, p, sink, noise_lanes);
                             if (r == kStepMoved) {
                                 ++my_events;

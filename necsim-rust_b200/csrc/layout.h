@@ -89,6 +89,9 @@ struct alignas(16) PoissonConsts {
 };
 static_assert(sizeof(PoissonConsts) % 16 == 0, "PoissonConsts must be whole 16-byte words");
 
+// SimParams.chain bits
+constexpr int32_t kChainPoisson = 1, kChainExp = 2;
+
 // Per-simulation scalars, read by every lineage of the simulation.
 struct alignas(16) SimParams {
     PoissonConsts pois;       // the samplers' constants under uniform turnover
@@ -135,7 +138,7 @@ struct alignas(16) SimParams {
     uint64_t step_slice_max;
     uint64_t lineage_offset;  // first slot of the simulation's resident-arena segment
     int32_t resident;         // 1 once the resident kernel owns the simulation
-    int32_t chain;            // 1: chain_run may step the simulation's lineages (kernels.cu)
+    int32_t chain;            // samplers whose lineages chain_run may step (kernels.cu)
     int32_t active;           // 1 while the simulation still advances
     int32_t pad;
 };
