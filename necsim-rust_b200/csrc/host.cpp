@@ -900,7 +900,7 @@ void choose_launch(Engine &E) {
     if (per_sm < 1) per_sm = 1;
     E.step_block = block;
     E.step_grid = E.args.grid_size ? E.args.grid_size : (unsigned)(per_sm * E.n_sms);
-    if (E.args.event_time_sampler != NECSIM_SAMPLER_EXP) {
+    {
         // One warp per lineage, for rounds of up to four lineages per
         // resident warp (9,472 with four blocks per SM).  The cooperative
         // kernel steps about 4e9 events per second whatever the round's size
@@ -911,7 +911,7 @@ void choose_launch(Engine &E) {
         // 580 / 578 ms, with the learned schedule 516 / 502 / 499 / 509 ms,
         // one SpatiallyImplicit run of 30,011 lineages 40 / 36 / 36 / 36 ms.
         int coop_per_sm = 0;
-        CK(coop_kernel_occupancy(E.kind, &coop_per_sm));
+        CK(coop_kernel_occupancy(E.kind, E.args.event_time_sampler == NECSIM_SAMPLER_EXP, &coop_per_sm));
         if (coop_per_sm < 1) coop_per_sm = 1;
         E.coop_grid = (unsigned)(coop_per_sm * E.n_sms);
         E.coop_max = (uint64_t)E.coop_grid * (kCoopBlock / 32) * 4;
@@ -1246,7 +1246,7 @@ FeatureArgs make_feature_args(Engine &E, DeviceLineages &in) {
     f.kind = E.kind;
     // rounds stepped one warp at a time per lineage (the cooperative kernel, or the
     // exponential sampler's step kernel when it has a warp per lineage)
-    f.skip_at_most = E.coop_max ? E.coop_max : (uint64_t)E.step_grid * (E.step_block / 32);
+    f.skip_at_most = E.coop_max;
     return f;
 }
 
@@ -1519,7 +1519,7 @@ RunResult run_rounds(Engine &E) {
             } else {
                 enqueue_rounds(E, rounds, true, false);
             }
-            rr.launches += (uint64_t)rounds * ((E.learned ? 9 : 5) + (E.coop_max ? 1 : 0));
+            rr.launches += (uint64_t)rounds * (E.learned ? 10 : 6);
             // after an even number of rounds the live lineages are in A
             if (E.tracing) CK(launch_trace_snapshot(make_feature_args(E, E.A), E.trace_snap++, E.trace_rows,
                                                     E.trace_counts, E.trace_rows_cap, E.stream));
@@ -2335,7 +2335,7 @@ void prepare_batch(BatchRun &b, std::vector<SimHost> sims, const necsim_args &ar
         // fit its cooperative kernel's warps on the reserved SMs
         if (reserved && role == kGateOnly) {
             int coop_per_sm = 0;
-            CK(coop_kernel_occupancy(E.kind, &coop_per_sm));
+            CK(coop_kernel_occupancy(E.kind, E.args.event_time_sampler == NECSIM_SAMPLER_EXP, &coop_per_sm));
             E.gate_lineages = (uint64_t)reserved * (uint64_t)std::max(coop_per_sm, 1) * (kCoopBlock / 32);
         }
         b.members.push_back(std::move(ids));

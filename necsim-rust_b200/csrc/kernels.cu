@@ -1075,7 +1075,10 @@ struct Chain {
 // EXP: the exponential sampler (exp.rs:37-83).  Lane (b, j) holds sample j of
 // bucket base + b, b < 4, and the event that it would be; every lane adds up
 // its bucket's samples in order (the reference's rounding) from the others'.
-// Times are not scaled: any delta_t.
+// Times are not scaled: any delta_t.  One lineage, select first and then work
+// the event out -> this form: NonSpatial 2,963 -> 1,481 cycles per event,
+// SpatiallyImplicit 3,037 -> 1,452, AlmostInfinite 2,858 -> 1,529,
+// SpatiallyExplicit 3,904 -> 3,215.
 constexpr int kFastNone = 0, kFastNormal = 1, kFastClark = 2;
 template <int KIND, bool LOCAL, bool EXP, int FAST = kFastNone>
 __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p, const EventSink &k,
@@ -1696,7 +1699,6 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
         const NoiseLane noise_lanes = noise_lane<KIND>(p);
         int r;
         if constexpr (EXP) {
-            uint32_t moved = 0;
             const bool chain = chain_takes<KIND, true>(p, c);
             if constexpr (kChainKind<KIND>) {
                 if (chain) r = chain_run<KIND, true>(c, p, sink, warp_steps);
@@ -1705,10 +1707,6 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
                 r = lineage_step_coop<KIND, true>(c, p, sink, noise_lanes);
                 if (r != kStepMoved) break;
                 warp_steps += 1;
-                if (++moved == a.slice) {
-                    r = kStepSlice;
-                    break;
-                }
             }
             if (!chain && r == kStepSpeciated) warp_steps += 1;
         } else {
@@ -1769,8 +1767,6 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
         if (lane_id == 0) {
             if (r == kStepStop)
                 store_stopped(a, c);
-            else if (r == kStepSlice)
-                store_sliced(a, c);
             else
                 a.state[c.slot] = (r == kStepSpeciated) ? 1 : 2;
         }
@@ -1793,27 +1789,18 @@ __device__ __forceinline__ void step_body(const StepArgs &a) {
     // one simulation: its parameters live in shared memory for the launch
     __shared__ __align__(16) unsigned char params_smem[SINGLE ? sizeof(SimParams) : 16];
     const uint64_t n = *a.n_cur;
-    // the Poisson sampler's cooperative rounds run in coop_kernel
-    if (n == 0 || (!EXP && n <= a.coop_max)) return;
+    // the cooperative rounds run in coop_kernel
+    if (n <= a.coop_max) return;
     // Only the blocks that a round can fill take part: consecutive blocks sit
     // on different SMs, while among all resident warps those of a quarter of
     // the SMs won the race for the queue (30,000 lineages: 26.6 warps active
     // on the busiest SM, 0.1 on the idlest).  30,000 lineages 3.5 -> 7.4e9
     // events per second, 46,000 5.4 -> 9.8e9.
-    // (a warp per lineage: the exponential sampler's sparse rounds, and all
-    // WrappingNoise ones)
-    const bool by_warp = EXP && (KIND == kWrappingNoise || n <= (uint64_t)gridDim.x * (blockDim.x / 32u));
-    const unsigned warps = by_warp ? warps_taking_part(a, n, blockDim.x / 32u) : 0u;
-    if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * (by_warp ? warps : blockDim.x) >= n) return;
+    if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * blockDim.x >= n) return;
     if (block_leaves(a.gate, a.gate_role, a.blocks_done)) return;
     const SimParams *P = stage_params<SINGLE>(a, params_smem);
     const EventSink sink = sink_of(a);
     const unsigned lane_id = threadIdx.x & 31u;
-    if (by_warp) {
-        if (threadIdx.x / 32u < warps) coop_body<KIND, SINGLE, true>(a, P, n);
-        block_arrives(a.gate, a.gate_role, a.blocks_done);
-        return;
-    }
     const bool lat = EXP && n * 4 <= (uint64_t)gridDim.x * blockDim.x;
     const unsigned lanemask_lt = (1u << lane_id) - 1u;
     bool have = false;
@@ -1893,12 +1880,18 @@ __global__ void __launch_bounds__(kStepBlockMax, 1) step_kernel_exp(StepArgs a) 
     step_body<KIND, SINGLE, true>(a);
 }
 
-// The Poisson sampler's rounds with at most coop_max live lineages, one warp
-// per lineage; the step kernel takes the other rounds.  Its own kernel, so
-// that the speculative form's registers do not lower the step kernel's
-// occupancy.
-template <int KIND, bool SINGLE>
-__global__ void __launch_bounds__(kCoopBlock) coop_kernel(StepArgs a) {
+// The rounds with at most coop_max live lineages, one warp per lineage; the
+// step kernel takes the others.  Its own kernel, so that the speculative
+// form's registers do not lower the step kernel's occupancy: with the
+// exponential sampler's rounds in step_kernel_exp that took 138 registers, in
+// this kernel it takes 100.  Exponential sampler, 10^6 NonSpatial lineages
+// 27.3 -> 23.7 ms, 30,011 SpatiallyImplicit ones 77 -> 70 ms, 32 SpatiallyImplicit
+// simulations 177 -> 151 ms; 10^5 NonSpatial ones the same.  Left to itself the
+// compiler keeps its chain within 128 registers, at 1,540 cycles per event
+// against 1,481 with 138 to 148; the Poisson sampler's 64-simulation sweep is
+// the slower one with more registers and fewer warps (494 -> 503 ms).
+template <int KIND, bool SINGLE, bool EXP>
+__global__ void __launch_bounds__(kCoopBlock, EXP ? 1 : 0) coop_kernel(StepArgs a) {
     __shared__ __align__(16) unsigned char params_smem[SINGLE ? sizeof(SimParams) : 16];
     const uint64_t n = *a.n_cur;
     if (n == 0 || n > a.coop_max) return;
@@ -1906,7 +1899,7 @@ __global__ void __launch_bounds__(kCoopBlock) coop_kernel(StepArgs a) {
     if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * warps >= n) return;
     if (block_leaves(a.gate, a.gate_role, a.blocks_done)) return;
     const SimParams *P = stage_params<SINGLE>(a, params_smem);
-    if (threadIdx.x / 32u < warps) coop_body<KIND, SINGLE, false>(a, P, n);
+    if (threadIdx.x / 32u < warps) coop_body<KIND, SINGLE, EXP>(a, P, n);
     block_arrives(a.gate, a.gate_role, a.blocks_done);
 }
 
@@ -2415,27 +2408,35 @@ __global__ void schedule_kernel(ScheduleArgs a) {
 }
 
 // ---- host-side launchers ----
+template <int KIND, bool EXP>
+static void launch_coop_t(const StepArgs &a, unsigned coop_grid, cudaStream_t st) {
+    if (a.n_sims == 1)
+        coop_kernel<KIND, true, EXP><<<coop_grid, kCoopBlock, 0, st>>>(a);
+    else
+        coop_kernel<KIND, false, EXP><<<coop_grid, kCoopBlock, 0, st>>>(a);
+}
+
 template <int KIND>
 static cudaError_t launch_step_t(const StepArgs &a, unsigned grid, unsigned block, unsigned coop_grid,
                                  cudaStream_t st) {
-    if (a.exp_sampler) {
-        if (a.n_sims == 1)
-            step_kernel_exp<KIND, true><<<grid, block, 0, st>>>(a);
-        else
-            step_kernel_exp<KIND, false><<<grid, block, 0, st>>>(a);
-        return cudaGetLastError();
-    }
     if (a.coop_max) {
-        if (a.n_sims == 1)
-            coop_kernel<KIND, true><<<coop_grid, kCoopBlock, 0, st>>>(a);
+        if (a.exp_sampler)
+            launch_coop_t<KIND, true>(a, coop_grid, st);
         else
-            coop_kernel<KIND, false><<<coop_grid, kCoopBlock, 0, st>>>(a);
+            launch_coop_t<KIND, false>(a, coop_grid, st);
     }
+    // (a WrappingNoise target takes a whole warp: every round is cooperative)
     if constexpr (KIND != kWrappingNoise) {
-        if (a.n_sims == 1)
+        if (a.exp_sampler) {
+            if (a.n_sims == 1)
+                step_kernel_exp<KIND, true><<<grid, block, 0, st>>>(a);
+            else
+                step_kernel_exp<KIND, false><<<grid, block, 0, st>>>(a);
+        } else if (a.n_sims == 1) {
             step_kernel<KIND, true><<<grid, block, 0, st>>>(a);
-        else
+        } else {
             step_kernel<KIND, false><<<grid, block, 0, st>>>(a);
+        }
     }
     return cudaGetLastError();
 }
@@ -2453,29 +2454,33 @@ cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned blo
 }
 
 template <int KIND>
-static cudaError_t coop_occupancy_t(int *blocks_per_sm) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, coop_kernel<KIND, false>, kCoopBlock, 0);
+static cudaError_t coop_occupancy_t(bool exp_sampler, int *blocks_per_sm) {
+    if (exp_sampler)
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, coop_kernel<KIND, false, true>, kCoopBlock,
+                                                             0);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, coop_kernel<KIND, false, false>, kCoopBlock, 0);
 }
 
-cudaError_t coop_kernel_occupancy(int kind, int *blocks_per_sm) {
+cudaError_t coop_kernel_occupancy(int kind, bool exp_sampler, int *blocks_per_sm) {
     switch (kind) {
-    case kNonSpatial: return coop_occupancy_t<kNonSpatial>(blocks_per_sm);
-    case kSpatiallyImplicit: return coop_occupancy_t<kSpatiallyImplicit>(blocks_per_sm);
-    case kAlmostInfiniteNormal: return coop_occupancy_t<kAlmostInfiniteNormal>(blocks_per_sm);
-    case kSpatiallyExplicit: return coop_occupancy_t<kSpatiallyExplicit>(blocks_per_sm);
-    case kWrappingNoise: return coop_occupancy_t<kWrappingNoise>(blocks_per_sm);
+    case kNonSpatial: return coop_occupancy_t<kNonSpatial>(exp_sampler, blocks_per_sm);
+    case kSpatiallyImplicit: return coop_occupancy_t<kSpatiallyImplicit>(exp_sampler, blocks_per_sm);
+    case kAlmostInfiniteNormal: return coop_occupancy_t<kAlmostInfiniteNormal>(exp_sampler, blocks_per_sm);
+    case kSpatiallyExplicit: return coop_occupancy_t<kSpatiallyExplicit>(exp_sampler, blocks_per_sm);
+    case kWrappingNoise: return coop_occupancy_t<kWrappingNoise>(exp_sampler, blocks_per_sm);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <int KIND>
 static cudaError_t step_occupancy_t(bool exp_sampler, int block, int *blocks_per_sm) {
-    if (exp_sampler)
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel_exp<KIND, false>, block, 0);
-    if constexpr (KIND == kWrappingNoise)
-        return coop_occupancy_t<KIND>(blocks_per_sm);
-    else
+    if constexpr (KIND == kWrappingNoise) {  // (no step kernel)
+        return coop_occupancy_t<KIND>(exp_sampler, blocks_per_sm);
+    } else {
+        if (exp_sampler)
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel_exp<KIND, false>, block, 0);
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<KIND, false>, block, 0);
+    }
 }
 
 cudaError_t step_kernel_occupancy(int kind, bool exp_sampler, int block, int *blocks_per_sm) {

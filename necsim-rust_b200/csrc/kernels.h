@@ -51,8 +51,7 @@ struct StepArgs {
     uint32_t n_sims;                     // simulations in `params`
     TraceSink trace;                     // death records of speciated lineages (tracing only)
     uint32_t exp_sampler;                // 1: exponential event-time sampler (exp.rs), else Poisson
-    // Poisson sampler: rounds with at most this many live lineages run in
-    // the cooperative kernel (one warp per lineage); 0: the step kernel takes
+    // rounds with at most this many live lineages run in the cooperative kernel (one warp per lineage); 0: the step kernel takes
     // every round (WrappingNoise: ~0, it takes none)
     uint64_t coop_max;
     uint32_t n_sms;                      // SMs the kernels' grids are spread over
@@ -109,14 +108,14 @@ struct ScheduleArgs {
     unsigned long long *rounds_seen;     // the most rounds that a simulation has begun
 };
 
-// the step kernel on grid x block and, for the Poisson sampler with
-// a.coop_max > 0, the cooperative kernel on coop_grid x kCoopBlock before it
+// the step kernel on grid x block and, with a.coop_max > 0, the cooperative
+// kernel on coop_grid x kCoopBlock before it
 // (WrappingNoise: every round runs there); each returns at once in the
 // other's rounds
 cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned block, unsigned coop_grid,
                         cudaStream_t st);
 cudaError_t step_kernel_occupancy(int kind, bool exp_sampler, int block, int *blocks_per_sm);
-cudaError_t coop_kernel_occupancy(int kind, int *blocks_per_sm);
+cudaError_t coop_kernel_occupancy(int kind, bool exp_sampler, int *blocks_per_sm);
 cudaError_t launch_dedup(const DedupArgs &a, unsigned grid, unsigned block, cudaStream_t st);
 cudaError_t launch_schedule(const ScheduleArgs &a, cudaStream_t st);
 

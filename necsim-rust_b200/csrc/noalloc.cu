@@ -223,7 +223,7 @@ extern "C" int necsim_gpu_round_noalloc(const necsim_scenario *scenario, const n
     int step_per_sm = 0, coop_per_sm = 0;
     if (step_kernel_occupancy(scenario->kind, exp_sampler, (int)kBlock, &step_per_sm) != cudaSuccess)
         return NECSIM_E_CUDA;
-    if (!exp_sampler && coop_kernel_occupancy(scenario->kind, &coop_per_sm) != cudaSuccess) return NECSIM_E_CUDA;
+    if (coop_kernel_occupancy(scenario->kind, exp_sampler, &coop_per_sm) != cudaSuccess) return NECSIM_E_CUDA;
     const unsigned step_grid = sms * (unsigned)(step_per_sm > 0 ? step_per_sm : 1);
     const unsigned coop_grid = sms * (unsigned)(coop_per_sm > 0 ? coop_per_sm : 1);
 
@@ -255,7 +255,7 @@ extern "C" int necsim_gpu_round_noalloc(const necsim_scenario *scenario, const n
     sa.n_sims = 1;
     sa.n_sms = sms;
     sa.exp_sampler = exp_sampler ? 1u : 0u;
-    sa.coop_max = exp_sampler ? 0 : (uint64_t)coop_grid * (kCoopBlock / 32) * 4;
+    sa.coop_max = (uint64_t)coop_grid * (kCoopBlock / 32) * 4;
     if (launch_step(scenario->kind, sa, step_grid, kBlock, coop_grid, st) != cudaSuccess) return NECSIM_E_CUDA;
 
     DedupArgs da;

@@ -214,3 +214,44 @@ def test_displacements_decided_in_32_bits(nb, syn, oracle, desc):
                         step_slice_max=1024)
     assert g.steps == c.steps > 500_000
     assert same_stream(g.speciation, c.speciation)
+
+
+EXP_CASES = sorted(n for n in CASES if CASES[n][2] is None) + ["explicit-" + n for n in sorted(SE_CASES)]
+
+
+@pytest.mark.parametrize("name", EXP_CASES)
+@pytest.mark.parametrize("batch", [False, True])
+def test_exponential_sampler(nb, syn, oracle, name, batch):
+    """The exponential sampler's form: buckets that hold many samples or whose
+    first sample is past the end, at the same edges."""
+    if name.startswith("explicit-"):
+        make, kw = SE_CASES[name[len("explicit-"):]]
+        desc = make(syn)
+    else:
+        desc, kw, _ = CASES[name]
+    nu = desc["speciation_probability"]
+    kw = dict(dict(delta_t=3.0), **kw)
+    algo = nb.CUDA(event_time_sampler="exp", resident=batch, **kw)
+    if batch:
+        g = nb.simulate_batch([syn.to_scenario(desc)] * 2, [nu, min(1.0, 2 * nu)], [5, 6], algo, collect=True)[0]
+    else:
+        with nb.Simulation(syn.to_scenario(desc), nu, algo) as sim:
+            g = sim.simulate(5)
+    oracle_kw = dict(dict(step_slice=10, min_round_events=1 << 20), **kw)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice_max=1024, event_time_sampler=oracle.SAMPLER_EXP,
+                        **oracle_kw)
+    assert g.steps == c.steps > 0
+    assert same_stream(g.speciation, c.speciation)
+    assert (g.n_rounds, g.n_dedup, g.time) == (c.n_rounds, c.n_dedup, c.time)
+
+
+@pytest.mark.parametrize("n", [147, 149, 1776, 1777, 7104, 7105, 9472, 9473])
+def test_exponential_round_sizes(nb, syn, oracle, n):
+    desc = ns(n, 1, 1, 0.05)
+    algo = nb.CUDA(event_time_sampler="exp", step_slice=2, min_round_events=1)
+    with nb.Simulation(syn.to_scenario(desc), 0.05, algo) as sim:
+        g = sim.simulate(5)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice_max=1024, step_slice=2, min_round_events=1,
+                        event_time_sampler=oracle.SAMPLER_EXP)
+    assert same_stream(g.speciation, c.speciation)
+    assert (g.steps, g.n_rounds, g.n_dedup, g.time) == (c.steps, c.n_rounds, c.n_dedup, c.time)
