@@ -663,6 +663,21 @@ struct Control {  // small device scalars
     unsigned int pad;
 };
 
+// Host memory for events, grown on demand and not zeroed.  Kept between calls
+// (up to EnginePool::kHostBytes): the page faults of fresh memory made 34 MB of
+// records take 14 ms to copy from the device instead of 1.5 ms.
+struct HostBuffer {
+    std::unique_ptr<unsigned char[]> data;
+    size_t bytes = 0;
+    void reserve(size_t need) {
+        if (bytes >= need) return;
+        bytes = 0;
+        data.reset();
+        data.reset(new unsigned char[need + need / 4]);
+        bytes = need + need / 4;
+    }
+};
+
 // Events delivered round by round (dispersal reporting): per simulation the
 // species counted so far and the last speciation event delivered.
 struct Delivery {
@@ -696,6 +711,8 @@ struct Engine {
     uint64_t n_cap = 0;
     unsigned char *sort_mem = nullptr;  // scratch of the event sort, grown on demand
     size_t sort_bytes = 0;
+    uint64_t references = 1;            // one above the usual global references
+    HostBuffer host_events[2];          // sorted speciation and dispersal events on the host
     uint64_t disp_room = 0;             // dispersal events that d_disp holds
     unsigned long long context = 0;     // CUDA context id while idle in the EnginePool
     DeviceLineages A, B;
@@ -789,6 +806,7 @@ struct Engine {
         if (sort_mem) cudaFree(sort_mem);
         arena = sort_mem = nullptr;
         arena_bytes = sort_bytes = 0;
+        for (auto &h : host_events) h = HostBuffer();
         drop_inputs();
         for (auto p : d_cells)
             if (p) cudaFree(p);
@@ -1570,35 +1588,6 @@ inline uint64_t bits_of(double v) {
     return b;
 }
 
-// PackedEvent::cmp (necsim/core/src/event.rs:256-280) for speciation events
-// (target == origin), per simulation.
-bool spec_less(const DevSpeciationEvent &a, const DevSpeciationEvent &b) {
-    if (a.sim != b.sim) return a.sim < b.sim;
-    const uint64_t ta = bits_of(a.event_time), tb = bits_of(b.event_time);
-    if (ta != tb) return ta < tb;
-    if (a.x != b.x) return a.x < b.x;
-    if (a.y != b.y) return a.y < b.y;
-    if (a.idx != b.idx) return a.idx < b.idx;
-    const uint64_t pa = bits_of(a.prior_time), pb = bits_of(b.prior_time);
-    if (pa != pb) return pa < pb;
-    return a.gref < b.gref;
-}
-
-bool disp_less(const DevDispersalEvent &a, const DevDispersalEvent &b) {
-    if (a.sim != b.sim) return a.sim < b.sim;
-    const uint64_t ta = bits_of(a.event_time), tb = bits_of(b.event_time);
-    if (ta != tb) return ta < tb;
-    if (a.x != b.x) return a.x < b.x;
-    if (a.y != b.y) return a.y < b.y;
-    if (a.idx != b.idx) return a.idx < b.idx;
-    if (a.tx != b.tx) return a.tx < b.tx;
-    if (a.ty != b.ty) return a.ty < b.ty;
-    if (a.tidx != b.tidx) return a.tidx < b.tidx;
-    const uint64_t pa = bits_of(a.prior_time), pb = bits_of(b.prior_time);
-    if (pa != pb) return pa < pb;
-    return a.gref < b.gref;
-}
-
 // PackedEvent::cmp (event.rs:256-280) between a speciation event (whose
 // target is its origin, event.rs:105-115) and a dispersal event of the same
 // simulation: event time, origin, target, prior time, global reference.
@@ -1617,29 +1606,35 @@ bool spec_before_disp(const DevSpeciationEvent &a, const DevDispersalEvent &b) {
 }
 
 // Event records from the device in PackedEvent order per simulation: sorted
-// by (simulation, event time) on the device, runs of equal times (and small
-// counts, or all when the scratch cannot be had) on the host.  A call with
-// ten million NonSpatial lineages (290,000 speciations) takes 65 ms with the
+// on the device, on the host small counts, all when the scratch cannot be
+// had, and runs of equal times that the device left unordered.  A call with
+// ten million NonSpatial lineages (290,000 speciations) took 65 ms with the
 // host's sort and 52 ms with the device's, one that reports 0.5 million
-// dispersal events 101 and 75 ms (the rest: some 5,000 reporter calls); below
-// kDeviceSort the 26 launches cost as much as the sort.
+// dispersal events 101 and 75 ms, and 35 ms with the ties ordered on the device
+// as well (and host memory that is kept).  kDeviceSort: a call with 8,191
+// records, sorted on the host, takes 1.03 ms and one with 8,192, sorted here,
+// 0.80 ms; the launches cost as much as the host's sort at about half as many.
 constexpr uint64_t kDeviceSort = 8192;
 
 template <typename Record>
-struct Fetched {
-    std::unique_ptr<Record[]> data;  // not zeroed
+struct Fetched {  // in the engine's host memory
+    Record *data = nullptr;
     uint64_t n = 0;
-    Record *begin() { return data.get(); }
-    Record *end() { return data.get() + n; }
+    Record *begin() { return data; }
+    Record *end() { return data + n; }
 };
 
-template <typename Record, typename Less>
-Fetched<Record> fetch_sorted(Engine &E, const Record *dev, uint64_t n, Less less) {
+// `slot`: which of the engine's host buffers holds the records.
+template <typename Record>
+Fetched<Record> fetch_sorted(Engine &E, int slot, const Record *dev, uint64_t n) {
     Fetched<Record> f;
     f.n = n;
     if (n == 0) return f;
-    f.data.reset(new Record[n]);
+    HostBuffer &host = E.host_events[slot];
+    host.reserve(n * sizeof(Record));
+    f.data = reinterpret_cast<Record *>(host.data.get());
     Record *from = nullptr;
+    uint32_t *dev_unordered = nullptr, unordered = 0;
     if (n >= kDeviceSort) {
         const size_t need = sort_scratch_bytes(n, sizeof(Record));
         if (E.sort_bytes < need) {
@@ -1656,15 +1651,20 @@ Fetched<Record> fetch_sorted(Engine &E, const Record *dev, uint64_t n, Less less
                 cudaGetLastError();  // sorted on the host instead
             }
         }
-        if (E.sort_mem)
-            CK(sort_records(dev, n, (uint32_t)E.sims.size(), E.sort_mem, E.aux_grid, &from, E.stream));
+        if (E.sort_mem) {
+            CK(sort_records(dev, n, (uint32_t)E.sims.size(), E.references, E.sort_mem, E.aux_grid, &from,
+                            &dev_unordered, E.stream));
+            CK(cudaMemcpyAsync(&unordered, dev_unordered, sizeof(unordered), cudaMemcpyDeviceToHost, E.stream));
+        }
     }
-    CK(cudaMemcpyAsync(f.begin(), from ? from : dev, n * sizeof(Record), cudaMemcpyDeviceToHost, E.stream));
+    CK(cudaMemcpyAsync(f.data, from ? from : dev, n * sizeof(Record), cudaMemcpyDeviceToHost, E.stream));
     CK(cudaStreamSynchronize(E.stream));
+    const auto less = [](const Record &a, const Record &b) { return event_less(a, b); };
     if (!from) {
         std::sort(f.begin(), f.end(), less);
         return f;
     }
+    if (!unordered) return f;
     for (Record *a = f.begin(); a != f.end();) {
         Record *b = a + 1;
         while (b != f.end() && b->sim == a->sim && bits_of(b->event_time) == bits_of(a->event_time)) ++b;
@@ -1688,13 +1688,15 @@ static_assert(sizeof(DevDispersalEvent) == sizeof(necsim_dispersal_event) &&
               "dispersal records are handed over in place");
 void deliver(const necsim_reporter *rep, DevSpeciationEvent *a, DevSpeciationEvent *b) {
     if (a == b || !rep || !rep->report_speciation) return;
-    for (DevSpeciationEvent *e = a; e != b; ++e) e->sim = 0;
+    if (a->sim != 0)
+        for (DevSpeciationEvent *e = a; e != b; ++e) e->sim = 0;
     if (rep->report_speciation(rep->user, reinterpret_cast<necsim_speciation_event *>(a), (uint64_t)(b - a)) != 0)
         fail(NECSIM_E_CALLBACK, "reporter stopped the delivery");
 }
 void deliver(const necsim_reporter *rep, DevDispersalEvent *a, DevDispersalEvent *b) {
     if (a == b || !rep || !rep->report_dispersal) return;
-    for (DevDispersalEvent *e = a; e != b; ++e) e->sim = 0;
+    if (a->sim != 0)
+        for (DevDispersalEvent *e = a; e != b; ++e) e->sim = 0;
     if (rep->report_dispersal(rep->user, reinterpret_cast<necsim_dispersal_event *>(a), (uint64_t)(b - a)) != 0)
         fail(NECSIM_E_CALLBACK, "reporter stopped the delivery");
 }
@@ -1707,8 +1709,8 @@ void drain_events(Engine &E) {
         fail(NECSIM_E_TOO_LARGE, "one round produced more dispersal events than the event buffer holds "
                                  "(lower min_round_events or batch fewer simulations)");
     const uint64_t nd = c.n_disp_total, nsp = std::min<uint64_t>(c.n_spec_total, E.spec_cap);
-    Fetched<DevSpeciationEvent> sp = fetch_sorted(E, E.d_spec, nsp, spec_less);
-    Fetched<DevDispersalEvent> di = fetch_sorted(E, E.d_disp, nd, disp_less);
+    Fetched<DevSpeciationEvent> sp = fetch_sorted(E, 0, E.d_spec, nsp);
+    Fetched<DevDispersalEvent> di = fetch_sorted(E, 1, E.d_disp, nd);
     E.d2h_bytes += sizeof(c) + nsp * sizeof(DevSpeciationEvent) + nd * sizeof(DevDispersalEvent);
     // the next round appends from the start of both buffers
     CK(cudaMemset(&E.d_ctl->n_spec_total, 0, sizeof(unsigned long long)));
@@ -1722,8 +1724,9 @@ void drain_events(Engine &E) {
         const necsim_reporter *rep = dv.reporters ? (dv.one_reporter ? dv.reporters : &dv.reporters[s]) : nullptr;
         DevSpeciationEvent *i_end = i;
         DevDispersalEvent *j_end = j;
-        while (i_end != sp.end() && i_end->sim == s) ++i_end;
-        while (j_end != di.end() && j_end->sim == s) ++j_end;
+        const auto of_s = [&](const auto &e) { return e.sim == s; };
+        i_end = std::partition_point(i, sp.end(), of_s);
+        j_end = std::partition_point(j, di.end(), of_s);
         while (i != i_end || j != j_end) {
             DevSpeciationEvent *i0 = i;
             for (; i != i_end && (j == j_end || spec_before_disp(*i, *j)); ++i) {
@@ -1736,7 +1739,8 @@ void drain_events(Engine &E) {
             }
             deliver(rep, i0, i);
             DevDispersalEvent *j0 = j;
-            while (j != j_end && (i == i_end || !spec_before_disp(*i, *j))) ++j;
+            j = i == i_end ? j_end
+                           : std::partition_point(j, j_end, [&](const auto &d) { return !spec_before_disp(*i, d); });
             dv.n_dispersal[s] += (uint64_t)(j - j0);
             deliver(rep, j0, j);
         }
@@ -1823,7 +1827,7 @@ void finish(Engine &E, const RunResult &rr, const necsim_reporter *reporters, bo
         });
 
     const uint64_t n_spec = std::min<uint64_t>(c.n_spec_total, E.spec_cap);
-    Fetched<DevSpeciationEvent> ev = fetch_sorted(E, E.d_spec, n_spec, spec_less);
+    Fetched<DevSpeciationEvent> ev = fetch_sorted(E, 0, E.d_spec, n_spec);
     E.d2h_bytes += ns * sizeof(SimCounters) + sizeof(Control) + n * (4 * 4 + 8 * 3) +
                    n_spec * sizeof(DevSpeciationEvent);
 
@@ -2027,6 +2031,10 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
     if (off >= 0xffffffffULL) fail(NECSIM_E_TOO_LARGE, "more than 2^32 - 1 lineages");
     E.sims = std::move(sims);
     E.n_total = off;
+    // origins are numbered from 0 in every simulation; given lineages as they come
+    E.references = 1;
+    for (const SimHost &sh : E.sims) E.references = std::max<uint64_t>(E.references, sh.n_origins);
+    if (given) E.references = 1ULL << 32;
     for (size_t s = 0; s < E.sims.size(); ++s) {
         SimHost &sh = E.sims[s];
         if (sh.sc.kind == NECSIM_SPATIALLY_EXPLICIT) {
@@ -2086,6 +2094,7 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
 // run writes its lineages, parameters and counters anew.
 struct EnginePool {
     static constexpr size_t kEngines = 4;
+    static constexpr size_t kHostBytes = 64 << 20;  // per host buffer of an idle engine
     std::mutex mu;
     std::vector<std::unique_ptr<Engine>> idle;
 
@@ -2153,6 +2162,8 @@ struct EnginePool {
         const size_t limit = byte_limit(e->device);
         if (id == 0 || e->args.schedule || e->bytes() > limit) return;
         e->context = id;
+        for (auto &h : e->host_events)
+            if (h.bytes > kHostBytes) h = HostBuffer();
         std::vector<std::unique_ptr<Engine>> gone;  // freed after the lock
         std::lock_guard<std::mutex> lock(mu);
         for (size_t j = 0; j < idle.size();) {

@@ -141,14 +141,17 @@ struct ResidentArgs {
     unsigned int *blocks_done;           // that have finished or left (both zero at launch)
 };
 
-// Sorts n event records by (simulation, event time), stable (sort.cu):
-// *sorted points to them in `scratch` (sort_scratch_bytes(n, record size)
-// bytes, 256-byte aligned).  n < 2^32.
+// Sorts n event records by (simulation, event time, prior time, reference),
+// n < 2^32 (sort.cu): *sorted points to them in `scratch`
+// (sort_scratch_bytes(n, record size) bytes, 256-byte aligned), **unordered
+// is 0 if that is event_less's order and 1 if events of one time are not in
+// it yet.  `references`: one above the largest global reference; references
+// beyond it may end up unordered.
 size_t sort_scratch_bytes(uint64_t n, size_t record);
-cudaError_t sort_records(const DevSpeciationEvent *rec, uint64_t n, uint32_t n_sims, void *scratch, unsigned grid,
-                         DevSpeciationEvent **sorted, cudaStream_t st);
-cudaError_t sort_records(const DevDispersalEvent *rec, uint64_t n, uint32_t n_sims, void *scratch, unsigned grid,
-                         DevDispersalEvent **sorted, cudaStream_t st);
+cudaError_t sort_records(const DevSpeciationEvent *rec, uint64_t n, uint32_t n_sims, uint64_t references, void *scratch,
+                         unsigned grid, DevSpeciationEvent **sorted, uint32_t **unordered, cudaStream_t st);
+cudaError_t sort_records(const DevDispersalEvent *rec, uint64_t n, uint32_t n_sims, uint64_t references, void *scratch,
+                         unsigned grid, DevDispersalEvent **sorted, uint32_t **unordered, cudaStream_t st);
 
 // The SM ids present on the device: bit smid of mask[smid / 32] is set by a
 // block that ran there (grid blocks of 32 threads; mask zeroed before).

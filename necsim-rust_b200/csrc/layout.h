@@ -12,6 +12,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 
 namespace necsim {
 
@@ -197,6 +198,46 @@ struct DevDispersalEvent {
     uint32_t tx, ty, tidx;
     uint32_t sim, pad;
 };
+
+// PackedEvent::cmp (necsim/core/src/event.rs:256-280) within a simulation:
+// event time, origin, target, prior time, global reference (a speciation's
+// target is its origin, event.rs:105-115).  Times are not negative: their
+// bit patterns are in order.
+#ifdef __CUDACC__
+#define NECSIM_ORDER_FN __host__ __device__ inline
+#else
+#define NECSIM_ORDER_FN inline
+#endif
+NECSIM_ORDER_FN uint64_t time_bits(double v) {
+    uint64_t b;
+    memcpy(&b, &v, 8);
+    return b;
+}
+NECSIM_ORDER_FN bool event_less(const DevSpeciationEvent &a, const DevSpeciationEvent &b) {
+    if (a.sim != b.sim) return a.sim < b.sim;
+    const uint64_t ta = time_bits(a.event_time), tb = time_bits(b.event_time);
+    if (ta != tb) return ta < tb;
+    if (a.x != b.x) return a.x < b.x;
+    if (a.y != b.y) return a.y < b.y;
+    if (a.idx != b.idx) return a.idx < b.idx;
+    const uint64_t pa = time_bits(a.prior_time), pb = time_bits(b.prior_time);
+    if (pa != pb) return pa < pb;
+    return a.gref < b.gref;
+}
+NECSIM_ORDER_FN bool event_less(const DevDispersalEvent &a, const DevDispersalEvent &b) {
+    if (a.sim != b.sim) return a.sim < b.sim;
+    const uint64_t ta = time_bits(a.event_time), tb = time_bits(b.event_time);
+    if (ta != tb) return ta < tb;
+    if (a.x != b.x) return a.x < b.x;
+    if (a.y != b.y) return a.y < b.y;
+    if (a.idx != b.idx) return a.idx < b.idx;
+    if (a.tx != b.tx) return a.tx < b.tx;
+    if (a.ty != b.ty) return a.ty < b.ty;
+    if (a.tidx != b.tidx) return a.tidx < b.tidx;
+    const uint64_t pa = time_bits(a.prior_time), pb = time_bits(b.prior_time);
+    if (pa != pb) return pa < pb;
+    return a.gref < b.gref;
+}
 
 // Device status word bits (set instead of trapping).
 enum : uint32_t {

@@ -77,3 +77,28 @@ def test_dispersal_stream(nb, syn, oracle, batch):
         assert e["event_time"][0] >= last
         last = e["event_time"][-1]
     assert (at["s"], at["d"]) == (len(g.speciation), len(g.dispersal))
+
+
+@pytest.mark.parametrize("shift", [0, 20, 33])
+def test_references_beyond_the_sorted_digits(nb, syn, oracle, shift):
+    """Lineages that share their places from the start report the same events
+    under references that differ in their low digits or only above them (the
+    host settles the latter)."""
+    desc = dict(kind=0, speciation_probability=0.01, width=20, height=7, deme=1)
+    n = 600
+    lins = np.zeros(n, dtype=nb.LINEAGE_DTYPE)
+    u = syn.splitmix64(3, 2 * n)
+    lins["x"] = u[:n] % np.uint64(20)
+    lins["y"] = u[n:] % np.uint64(7)
+    lins["gref"] = np.arange(n, 0, -1, dtype=np.uint64) << np.uint64(shift)
+    with nb.Simulation(syn.to_scenario(desc), 0.01, nb.CUDA(report_dispersal=True, step_slice=60)) as sim:
+        g = sim.resume(lins, 0.0, 5)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, lineages=lins, step_slice=60, min_round_events=1 << 20,
+                        step_slice_max=1024, report_dispersal=True, dispersal_cap=1 << 20)
+    assert same_stream(g.speciation, c.speciation)
+    assert len(g.dispersal) == len(c.dispersal) > 10000
+    want = c.dispersal[packed_order(c.dispersal)]
+    t = want["event_time"]
+    assert (t[1:] == t[:-1]).sum() > 1000
+    for f in ("gref", "prior_time", "event_time", "x", "y", "index", "tx", "ty", "tindex"):
+        assert np.array_equal(g.dispersal[f], want[f]), f
