@@ -1050,6 +1050,16 @@ __device__ __forceinline__ void chain_unpack(const SimParams &p, uint64_t loc_te
     y = c.oy + row;
 }
 
+// An alias atom that is not kept in L1, for the map's cell records to stay
+// there: one SpatiallyExplicit lineage on dense maps of 8 / 16 / 24 / 32 / 48
+// cells squared 1,115 / 1,413 / 1,505 / 1,559 / 1,635 cycles per event with
+// the atoms in L1 and 1,436 / 1,463 / 1,485 / 1,486 / 1,536 past it; tables
+// of at most 1 MiB (kAtomsInL1) are read through it.
+__device__ __forceinline__ AliasAtom load_atom_past_l1(const AliasAtom *atom) {
+    const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(atom));
+    return {__hiloint2double((int)w.y, (int)w.x), w.z, w.w};
+}
+
 // A lineage between the events of chain_run.
 struct Chain {
     uint64_t loc_term;
@@ -1072,14 +1082,23 @@ struct Chain {
 // FAST: AlmostInfinite targets in 32-bit arithmetic where that decides them
 // (kFastNormal and kFastClark are loops of their own: together, one lineage
 // took 804 and 888 cycles per event).
+// FAST of SpatiallyExplicit: kFastNone lets every lane read its own
+// candidate's alias atom and target record while the search is decided (read
+// after the selection an event took 3,019 cycles), kSelected only the
+// selected lane.  32 random atoms of a table that L2 does not hold take as
+// long as the slowest of them: maps of 40 / 48 / 56 / 64 cells squared (31, 61,
+// 113 and 193 MB) 1,493 / 1,536 / 1,890 / 2,178 cycles with every lane's read and
+// 1,628 / 1,694 / 1,737 / 1,881 with one, so tables above 64 MiB, half of L2
+// (kSelectedAtoms), take the latter.
 // EXP: the exponential sampler (exp.rs:37-83).  Lane (b, j) holds sample j of
 // bucket base + b, b < 4, and the event that it would be; every lane adds up
 // its bucket's samples in order (the reference's rounding) from the others'.
 // Times are not scaled: any delta_t.  One lineage, select first and then work
 // the event out -> this form: NonSpatial 2,963 -> 1,481 cycles per event,
 // SpatiallyImplicit 3,037 -> 1,452, AlmostInfinite 2,858 -> 1,529,
-// SpatiallyExplicit 3,904 -> 3,215.
-constexpr int kFastNone = 0, kFastNormal = 1, kFastClark = 2;
+// SpatiallyExplicit 3,904 -> 3,215 (now 2,879, kSelected).
+constexpr int kFastNone = 0, kFastNormal = 1, kFastClark = 2, kSelected = 3;
+constexpr uint64_t kSelectedAtoms = 1 << 22, kAtomsInL1 = 1 << 16;
 template <int KIND, bool LOCAL, bool EXP, int FAST = kFastNone>
 __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p, const EventSink &k,
                                            const volatile unsigned *stop) {
@@ -1131,6 +1150,7 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
     const double horizon = EXP ? l.horizon : __dmul_rn(l.horizon, p.inv_delta_t);
     const float sigma_f = (float)sigma, shape_f = (float)p.clark_shape_u, exponent_f = (float)p.clark_exponent;
     const bool clark = p.clark != 0;
+    const bool past_l1 = FAST == kSelected || p.n_atoms > kAtomsInL1;
 
     constexpr uint32_t kFlush = 1u << 30;  // `moved` is added up before it overflows
     uint64_t tk = 0, search_k = 0, start_bits = 0;
@@ -1163,20 +1183,9 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
             // speciates and draws a migration test before its target
             // (dispersal_sampler/spatially_implicit.rs:58-86)
             leave = (kMigrates ? d2 : d1) <= leave_at_most;
-            uint64_t inj_k;
-            if constexpr (KIND == kAlmostInfiniteNormal) {
-                if (FAST == kFastNormal)
-                    leave = !normal_dispersal_fast(d2, d3, sigma_f, c.x, c.y, tx, ty) || leave;
-                else if (FAST == kFastClark)
-                    leave = !clark2dt_dispersal_fast(d2, d3, shape_f, exponent_f, c.x, c.y, tx, ty) || leave;
-                else
-                    normal_dispersal_draw(d2, d3, sigma, c.x, c.y, tx, ty);  // (Clark2Dt is always fast)
-                inj_k = (((uint64_t)ty << 32) | (uint64_t)tx) * kSeaHashK;
-            } else if constexpr (KIND == kSpatiallyExplicit) {
+            auto explicit_candidate = [&]() -> uint64_t {
                 // packed_separable_alias/dispersal.rs:16-77 (the cases of
-                // spatially_explicit_dispersal_draw): each lane reads its own
-                // candidate's alias atom and target record, while the search
-                // is decided (read after the selection an event took 3,019 cycles)
+                // spatially_explicit_dispersal_draw): the lane's own candidate
                 const double sd = c.rec.self_dispersal;
                 const bool stays = sd == 1.0, plain = sd == 0.0 || c.rec.non_self_event != c.cell;
                 const bool alias = !stays && (plain || __dmul_rn(v2, 0x1p-53) >= sd);
@@ -1192,11 +1201,11 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
                     if (at_cell >= c.rec.atom_count || at >= p.n_atoms) {
                         err = kErrAtomIndex;
                     } else {
-                        const AliasAtom atom = p.atoms[at];
+                        const AliasAtom atom = past_l1 ? load_atom_past_l1(p.atoms + at) : p.atoms[at];
                         target = frac < atom.u ? atom.e : atom.k;
                     }
                 }
-                inj_k = 0;
+                uint64_t inj_k = 0;
                 if (target >= p.n_cells) err |= kErrCellIndex;
                 if (err == 0) {
                     const CellRecord &there = p.cells[target];
@@ -1205,13 +1214,26 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
                 }
                 tx = target;
                 leave = leave || err != 0;
+                return inj_k;
+            };
+            uint64_t inj_k;
+            if constexpr (KIND == kAlmostInfiniteNormal) {
+                if (FAST == kFastNormal)
+                    leave = !normal_dispersal_fast(d2, d3, sigma_f, c.x, c.y, tx, ty) || leave;
+                else if (FAST == kFastClark)
+                    leave = !clark2dt_dispersal_fast(d2, d3, shape_f, exponent_f, c.x, c.y, tx, ty) || leave;
+                else
+                    normal_dispersal_draw(d2, d3, sigma, c.x, c.y, tx, ty);  // (Clark2Dt is always fast)
+                inj_k = (((uint64_t)ty << 32) | (uint64_t)tx) * kSeaHashK;
+            } else if constexpr (KIND == kSpatiallyExplicit) {
+                inj_k = FAST == kSelected ? 0ULL : explicit_candidate();
             } else {
                 const uint32_t cell = floor_u32(__dmul_rn(kMigrates ? v3 : v2, cells_u));
                 const uint32_t i = floor_u32(__dmul_rn(kMigrates ? v4 : v3, deme_u));
                 inj_k = (uint64_t)cell * deme_k + (uint64_t)i * kSeaHashK;
             }
-            loc_next = swap_halves(seahash_finish(inj_k)) ^ seed_term;
-            const uint32_t next_hi = leave ? kAttention : (uint32_t)(loc_next >> 32);
+            loc_next = FAST == kSelected ? 0ULL : swap_halves(seahash_finish(inj_k)) ^ seed_term;
+            uint32_t next_hi = leave ? kAttention : (uint32_t)(loc_next >> 32);
 
             if constexpr (EXP) {
                 // this lane's sample, and the running sum up to it
@@ -1268,6 +1290,11 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
                 sel = __reduce_min_sync(kFull, found ? key : kSelNone);
             }
 
+            if (FAST == kSelected && (lane == (sel & 31u) || (sel & kSelMore) != 0u || c.moved == attend)) {
+                const uint64_t inj_k = explicit_candidate();
+                loc_next = swap_halves(seahash_finish(inj_k)) ^ seed_term;
+                next_hi = leave ? kAttention : (uint32_t)(loc_next >> 32);
+            }
             const double q = __shfl_sync(kFull, mine, (int)(sel >> 20));
             const uint32_t lo = __shfl_sync(kFull, (uint32_t)loc_next, (int)sel);
             const uint32_t hi = __shfl_sync(kFull, next_hi, (int)sel);
@@ -1366,7 +1393,7 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
         if (leaves && !kMigrates && (!FAST || __shfl_sync(kFull, d1 <= leave_at_most ? 1 : 0, (int)cand)))
             return kStepSpeciated;
         if (k.report_dispersal && lane == 0) chain_unpack<KIND>(p, c.loc_term, LOCAL, c.cell, l.x, l.y, l.i);
-        if (FAST && leaves) {
+        if (KIND == kAlmostInfiniteNormal && FAST && leaves) {
             const uint64_t s_e = __shfl_sync(kFull, s, (int)cand);
             const uint64_t d2 = draw_at(s_e, 2), d3 = draw_at(s_e, 3);
             if (clark)
@@ -1439,8 +1466,10 @@ __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const Even
         result = chain_phase<KIND, true, EXP>(c, l, p, k, stop);
         c.local = result != kStepMoved;
     }
-    constexpr bool kPlane = KIND == kAlmostInfiniteNormal;
-    if (kPlane && p.clark)
+    constexpr bool kPlane = KIND == kAlmostInfiniteNormal, kMap = KIND == kSpatiallyExplicit;
+    if (kMap && p.n_atoms > kSelectedAtoms)
+        result = chain_phase<KIND, true, EXP, kMap ? kSelected : kFastNone>(c, l, p, k, stop);
+    else if (kPlane && p.clark)
         result = chain_phase<KIND, true, EXP, kPlane ? kFastClark : kFastNone>(c, l, p, k, stop);
     else if (kPlane && p.sigma <= kFastSigma)
         result = chain_phase<KIND, true, EXP, kPlane ? kFastNormal : kFastNone>(c, l, p, k, stop);

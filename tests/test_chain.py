@@ -255,3 +255,27 @@ def test_exponential_round_sizes(nb, syn, oracle, n):
                         event_time_sampler=oracle.SAMPLER_EXP)
     assert same_stream(g.speciation, c.speciation)
     assert (g.steps, g.n_rounds, g.n_dedup, g.time) == (c.steps, c.n_rounds, c.n_dedup, c.time)
+
+
+@pytest.mark.parametrize("side", [45, 46])
+@pytest.mark.parametrize("sampler", ["poisson", "exp"])
+def test_explicit_table_sizes(nb, syn, oracle, side, sampler):
+    """2025^2 and 2116^2 alias atoms: either side of the table size above which
+    only the selected lane reads its atom.  (The tests above have tables on
+    either side of the size that is read through L1.)"""
+    desc = se(syn, side, side, 4.0, 0.02, cell=1, p_zero=0.0)
+    desc["habitat"] = np.ones_like(desc["habitat"])
+    desc["dispersal"] = np.ones((side * side, side * side))
+    with nb.Simulation(syn.to_scenario(desc), 0.02, nb.CUDA(event_time_sampler=sampler, report_dispersal=True)) as sim:
+        g = sim.simulate(5)
+    c = oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, step_slice=10, min_round_events=1 << 20,
+                        step_slice_max=1024, report_dispersal=True, dispersal_cap=1 << 20,
+                        event_time_sampler=oracle.SAMPLER_EXP if sampler == "exp" else oracle.SAMPLER_POISSON)
+    assert g.steps == c.steps > 50_000
+    assert same_stream(g.speciation, c.speciation)
+    a = np.sort(g.dispersal, order=("event_time", "gref"))
+    b = np.sort(c.dispersal, order=("event_time", "gref"))
+    for f in ("gref", "prior_time", "event_time", "x", "y", "index", "tx", "ty", "tindex"):
+        assert np.array_equal(a[f], b[f]), f
+    with nb.Simulation(syn.to_scenario(desc), 0.02, nb.CUDA(event_time_sampler=sampler)) as sim:
+        assert same_stream(sim.simulate(5).speciation, c.speciation)
