@@ -964,22 +964,24 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
 //    Speciations, horizons, migrations and the rarer selections leave it
 //    with the event computed.
 // Measured with one lineage on a B200 (1,965 MHz), coop_run -> chain_run:
-// NonSpatial 1,772 -> 673 cycles per event, SpatiallyImplicit 1,747 -> 663,
-// AlmostInfinite Normal 2,793 -> 731, Clark2Dt 3,376 -> 725 (1,503 and 2,173
-// with f64 displacements), SpatiallyExplicit 3,019 -> 2,341 (64 x 64
-// map; its atoms, 190 MB, come from HBM).  The bound is the instruction count: a
+// NonSpatial 1,772 -> 652 cycles per event, SpatiallyImplicit 1,747 -> 650,
+// AlmostInfinite Normal 2,793 -> 701, Clark2Dt 3,376 -> 725 (1,503 and 2,173
+// with f64 displacements), SpatiallyExplicit 3,020 -> 1,898 (64 x 64
+// map; its atoms, 193 MB, come from HBM).  The bound is the instruction count: a
 // lone warp issues one instruction every two cycles, and NonSpatial takes 329
 // per event (48 a prime, 31 a sample).
 template <int KIND>
 constexpr bool kChainKind = KIND != kWrappingNoise;
 
 // Whether chain_run takes the simulation's round: SimParams.chain (for the
-// Poisson sampler delta_t a power of two, every table length below 2^32, no metacommunity cell inside
-// the local community) and time buckets that are exact doubles.
+// Poisson sampler delta_t a power of two, every table length below 2^32, no
+// metacommunity cell inside the local community) and time buckets that are
+// exact doubles.
 template <int KIND, bool EXP>
 __device__ __forceinline__ bool chain_takes(const SimParams &p, const Lane &l) {
     const double most = __dmul_rn(p.delta_t, 0x1p50);
-    return kChainKind<KIND> && (p.chain & (EXP ? kChainExp : kChainPoisson)) != 0 && l.horizon < most && l.last < most && p.min_event_time < most;
+    return kChainKind<KIND> && (p.chain & (EXP ? kChainExp : kChainPoisson)) != 0 && l.horizon < most &&
+           l.last < most && p.min_event_time < most;
 }
 
 // A bucket lane's search result, one word that orders by bucket: buckets
@@ -1237,8 +1239,7 @@ __device__ __forceinline__ int chain_phase(Chain &c, Lane &l, const SimParams &p
 
             if constexpr (EXP) {
                 // this lane's sample, and the running sum up to it
-                const double e =
-                    exp_sample(draw_at(primed_state_k(c.loc_term, search_k) + my_sample, 0), *pc);
+                const double e = exp_sample(draw_at(primed_state_k(c.loc_term, search_k) + my_sample, 0), *pc);
                 const double bucket = __dsub_rn(__longlong_as_double((long long)start_bits), 0x1p52);
                 const double slice_end = __dmul_rn(__dadd_rn(bucket, 1.0), delta_t);
                 double before_mine = c.before;  // the sum before this lane's sample (the first: nothing passed)
