@@ -884,7 +884,8 @@ void upload_tables(Engine &E, SimHost &s) {
         for (uint64_t c = 0; c < cells; ++c) tc[c] = make_poisson_consts(s.sc.turnover_map[c], s.params.delta_t);
         PoissonConsts *dt = dev_alloc<PoissonConsts>(cells);
         E.d_turnover.push_back(dt);
-        CK(cudaMemcpy(dt, tc.data(), cells * sizeof(PoissonConsts), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(dt, tc.data(), cells * sizeof(PoissonConsts), cudaMemcpyHostToDevice, E.stream));
+        CK(cudaStreamSynchronize(E.stream));  // tc goes
         E.h2d_bytes += cells * sizeof(PoissonConsts);
         s.params.turnover_cells = dt;
     }
@@ -1704,7 +1705,8 @@ void deliver(const necsim_reporter *rep, DevDispersalEvent *a, DevDispersalEvent
 void drain_events(Engine &E) {
     Delivery &dv = *E.delivery;
     Control c;
-    CK(cudaMemcpy(&c, E.d_ctl, sizeof(c), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(&c, E.d_ctl, sizeof(c), cudaMemcpyDeviceToHost, E.stream));
+    CK(cudaStreamSynchronize(E.stream));
     if (c.n_disp_total > E.disp_cap || (c.status & kErrDispersalOverflow))
         fail(NECSIM_E_TOO_LARGE, "one round produced more dispersal events than the event buffer holds "
                                  "(lower min_round_events or batch fewer simulations)");
@@ -1712,9 +1714,11 @@ void drain_events(Engine &E) {
     Fetched<DevSpeciationEvent> sp = fetch_sorted(E, 0, E.d_spec, nsp);
     Fetched<DevDispersalEvent> di = fetch_sorted(E, 1, E.d_disp, nd);
     E.d2h_bytes += sizeof(c) + nsp * sizeof(DevSpeciationEvent) + nd * sizeof(DevDispersalEvent);
-    // the next round appends from the start of both buffers
-    CK(cudaMemset(&E.d_ctl->n_spec_total, 0, sizeof(unsigned long long)));
-    CK(cudaMemset(&E.d_ctl->n_disp_total, 0, sizeof(unsigned long long)));
+    // the next round appends from the start of both buffers.  On the engine's
+    // stream: it is non-blocking, and a reset on the default stream may run
+    // after that round has counted events
+    CK(cudaMemsetAsync(&E.d_ctl->n_spec_total, 0, sizeof(unsigned long long), E.stream));
+    CK(cudaMemsetAsync(&E.d_ctl->n_disp_total, 0, sizeof(unsigned long long), E.stream));
     // per simulation: one stream in PackedEvent order, consecutive events of
     // one kind delivered in one call
     DevSpeciationEvent *i = sp.begin();
@@ -2238,7 +2242,7 @@ uint32_t reserve_sms(SmGate *gate, int device, int n_sms, uint32_t count) {
     CK(cudaSetDevice(device));
     SmGate g;
     std::memset(&g, 0, sizeof(g));
-    CK(cudaMemset(gate, 0, sizeof(SmGate)));
+    CK(cudaMemsetAsync(gate, 0, sizeof(SmGate), 0));
     CK(launch_sm_census(gate->mask, (unsigned)n_sms * 16u, 0));
     CK(cudaMemcpy(g.mask, gate->mask, sizeof(g.mask), cudaMemcpyDeviceToHost));
     std::vector<uint32_t> present;
@@ -2255,7 +2259,8 @@ uint32_t reserve_sms(SmGate *gate, int device, int n_sms, uint32_t count) {
         }
     }
     g.on = 0;
-    CK(cudaMemcpy(gate, &g, sizeof(g), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(gate, &g, sizeof(g), cudaMemcpyHostToDevice, 0));
+    CK(cudaStreamSynchronize(0));  // the engines' streams do not wait for it
     return n;
 }
 
@@ -2695,7 +2700,7 @@ int necsim_gpu_displacements(int32_t device, int32_t kind, const uint64_t *draws
         r.d = dev_alloc<uint64_t>(2 * n);
         r.x = dev_alloc<double>(n);
         r.y = dev_alloc<double>(n);
-        CK(cudaMemcpy(r.d, draws, 2 * n * sizeof(uint64_t), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(r.d, draws, 2 * n * sizeof(uint64_t), cudaMemcpyHostToDevice, 0));
         // the step kernels take the Clark2Dt exponent 1 / p computed on the host
         const double bb = kind == NECSIM_ALMOST_INFINITE_CLARK2DT ? 1.0 / b : 0.0;
         const int32_t dev_kind = kind == NECSIM_ALMOST_INFINITE_NORMAL ? (int32_t)kAlmostInfiniteNormal : -1;
