@@ -1460,7 +1460,11 @@ RunResult run_rounds(Engine &E) {
     CK(cudaMemcpyAsync(E.h_ctl, E.d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, E.stream));
     CK(cudaStreamSynchronize(E.stream));
     uint64_t enqueued = 0;
-    uint64_t stalled = 0;
+    // Rounds without an event or a merge before a run counts as hung.  A valid
+    // run passes through such rounds: until the horizon reaches the resume
+    // time, or while the last lineages sit in a turnover map's slow cells.
+    const uint64_t most_idle = 64ULL * graph_rounds;
+    uint64_t idle_rounds = 0, last_rounds = 0;
     unsigned long long last_steps = ~0ULL, last_live = ~0ULL;
     // one block per resident simulation, at most two per SM
     // at most one block per SM beside the global rounds (room for their
@@ -1475,9 +1479,6 @@ RunResult run_rounds(Engine &E) {
     // resident launch is in flight.
     bool res_inflight = false;
     while (E.h_ctl->n_active > 0 || E.h_ctl->n_resident > 0 || res_inflight) {
-        // every round advances each active simulation's horizon by at least
-        // step_slice / lambda, so each live lineage expects >= step_slice
-        // events per round: a valid run never reaches these bounds
         if (E.h_ctl->rounds_seen > max_rounds) fail(NECSIM_E_TIMEOUT, "round limit reached (necsim_args.max_rounds)");
         if (E.lazy_graph && !E.delivery && enqueued) {
             rounds = (unsigned)std::min<uint64_t>(graph_rounds, enqueued);  // 2, 2, 4, 8, ...
@@ -1485,13 +1486,16 @@ RunResult run_rounds(Engine &E) {
         }
         enqueued += rounds;
         if (E.h_ctl->steps_total == last_steps && E.h_ctl->n_cur == last_live && !res_inflight) {
-            if (++stalled >= 64) fail(NECSIM_E_TIMEOUT, "no progress over 64 graph launches");
+            idle_rounds += last_rounds;
+            if (idle_rounds >= most_idle)
+                fail(NECSIM_E_TIMEOUT, "no progress over " + std::to_string(idle_rounds) + " rounds");
         } else {
-            stalled = 0;
+            idle_rounds = 0;
         }
         last_steps = E.h_ctl->steps_total;
         last_live = E.h_ctl->n_cur;
         const bool global = E.h_ctl->n_active > 0;
+        last_rounds = global ? rounds : graph_rounds;
         if (E.args.resident) {
             if (res_inflight && cudaEventQuery(E.ev_res1) == cudaSuccess) {
                 float ms = 0.f;
