@@ -142,9 +142,10 @@ typedef struct necsim_args {
     struct necsim_model *model; /* schedule == 1: the lifetime model ordering the step queue
                                    (must stay alive during the call; same device) */
     uint64_t max_rounds;       /* watchdog: a run that needs more rounds fails with
-                                  NECSIM_E_TIMEOUT; 0 = default 2^26.  Every round advances each
-                                  live lineage by >= step_slice expected events, so a valid run
-                                  only meets a limit chosen below its round count */
+                                  NECSIM_E_TIMEOUT; 0 = default 2^26.  Counted in whole graphs of
+                                  rounds_per_graph, and only the rounds that the host launches: not
+                                  those that a lone lineage or a resident simulation runs by itself.
+                                  A valid run only meets a limit chosen below its round count */
     uint32_t priority_sims;    /* batches: this many simulations run in one priority engine (own
                                   rounds, stream and host thread) beside the others, so the others'
                                   rounds never hold them back: those in priority_list, else (schedule

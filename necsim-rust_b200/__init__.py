@@ -427,7 +427,8 @@ class CUDA:
     # algorithm's (event_time_sampler/exp.rs), -ln(U(0,1]) / lambda per event
     event_time_sampler: str = "poisson"
     # watchdog: a run still active after this many rounds fails with
-    # NECSIM_E_TIMEOUT (checked between graph launches); 0: 2^26
+    # NECSIM_E_TIMEOUT (whole graphs; not the rounds that a lone lineage or a
+    # resident simulation runs by itself); 0: 2^26
     max_rounds: int = 0
     # batches: simulations run in one priority engine beside the others
     # (their own rounds); `priority_list` names them (batch indices), else the

@@ -652,7 +652,7 @@ struct DeviceLineages {
 
 struct Control {  // small device scalars
     unsigned long long n_cur, out_count, work, mask, n_spec_total, n_disp_total, steps_total, visits;
-    unsigned long long rounds_seen;  // the most rounds that a simulation has begun
+    unsigned long long rounds_seen;  // the most rounds scheduled for a simulation by the schedule kernel
     unsigned int n_active;    // active simulations in the global rounds
     uint32_t status;
     unsigned int n_resident;  // active simulations owned by the resident kernel
@@ -1314,7 +1314,6 @@ ResidentArgs make_resident_args(Engine &E, uint32_t budget, const int *stop_flag
     a.steps_total = &E.d_ctl->steps_total;
     a.visits = &E.d_ctl->visits;
     a.n_resident = &E.d_ctl->n_resident;
-    a.rounds_seen = &E.d_ctl->rounds_seen;
     a.stop_flag = stop_flag;
     a.exp_sampler = E.args.event_time_sampler == NECSIM_SAMPLER_EXP ? 1u : 0u;
     a.gate = E.gate;
@@ -1469,7 +1468,6 @@ RunResult run_rounds(Engine &E) {
     // one block per resident simulation, at most two per SM
     // at most one block per SM beside the global rounds (room for their
     // kernels), two per SM when only resident simulations are left
-    const uint64_t max_rounds = E.args.max_rounds ? E.args.max_rounds : (1ULL << 26);
     const unsigned grid_beside = (unsigned)std::min<size_t>(E.sims.size(), (size_t)E.n_sms);
     const unsigned grid_alone = (unsigned)std::min<size_t>(E.sims.size(), (size_t)E.n_sms * 2);
     // The resident kernel runs on its own stream, decoupled from the global
@@ -1478,8 +1476,18 @@ RunResult run_rounds(Engine &E) {
     // over (promote) on the main stream, between graphs, only while no
     // resident launch is in flight.
     bool res_inflight = false;
+    // The round limit, in whole graphs: the rounds scheduled from here (a
+    // launch may run many rounds of a lone lineage, which are not counted) and
+    // the waits for the resident kernel.
+    const uint64_t max_rounds = E.args.max_rounds ? E.args.max_rounds : (1ULL << 26);
+    const uint64_t graph_limit = max_rounds / graph_rounds + (max_rounds % graph_rounds ? 1 : 0);
+    uint64_t resident_waits = 0;
+    auto check_round_limit = [&] {
+        if ((E.h_ctl->rounds_seen + resident_waits + graph_rounds - 1) / graph_rounds > graph_limit)
+            fail(NECSIM_E_TIMEOUT, "round limit reached (necsim_args.max_rounds)");
+    };
     while (E.h_ctl->n_active > 0 || E.h_ctl->n_resident > 0 || res_inflight) {
-        if (E.h_ctl->rounds_seen > max_rounds) fail(NECSIM_E_TIMEOUT, "round limit reached (necsim_args.max_rounds)");
+        check_round_limit();
         if (E.lazy_graph && !E.delivery && enqueued) {
             rounds = (unsigned)std::min<uint64_t>(graph_rounds, enqueued);  // 2, 2, 4, 8, ...
             if (!E.graph_exec && enqueued >= kGraphAfter) build_graph(E);
@@ -1550,6 +1558,7 @@ RunResult run_rounds(Engine &E) {
         } else if (res_inflight) {
             // only resident simulations are left: wait for their launch
             CK(cudaEventSynchronize(E.ev_res1));
+            resident_waits += 1;
         }
         CK(cudaMemcpyAsync(E.h_ctl, E.d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, E.stream));
         E.d2h_bytes += sizeof(Control);
@@ -1568,6 +1577,8 @@ RunResult run_rounds(Engine &E) {
             E.gate_on = true;
         }
     }
+    // (its last rounds may have begun since the last check)
+    if (!(E.h_ctl->status & ~kErrDedupFull)) check_round_limit();
     if (res_inflight) CK(cudaEventSynchronize(E.ev_res1));
     if (gate_owner) {
         // the other engines get every SM back

@@ -2170,8 +2170,6 @@ __global__ void __launch_bounds__(THREADS, 1) resident_kernel(ResidentArgs a) {
                 if (next_horizon(pm, n, h)) {
                     pm.horizon = h;
                     c.n_rounds += 1;
-                    if (c.n_rounds > *(volatile const unsigned long long *)a.rounds_seen)
-                        atomicMax(a.rounds_seen, c.n_rounds);
                     s_h = h;
                     s_go = 1;
                     // the global rounds running beside this launch have
@@ -2405,8 +2403,9 @@ __global__ void schedule_kernel(ScheduleArgs a) {
         if (more) {
             p.horizon = h;
             c.n_rounds += 1;
-            if (a.rounds_seen && c.n_rounds > *(volatile const unsigned long long *)a.rounds_seen)
-                atomicMax(a.rounds_seen, c.n_rounds);
+            c.n_scheduled += 1;
+            if (a.rounds_seen && c.n_scheduled > *(volatile const unsigned long long *)a.rounds_seen)
+                atomicMax(a.rounds_seen, c.n_scheduled);
         }
         p.active = more ? 1 : 0;
         if (c.routed) {

@@ -105,7 +105,7 @@ struct ScheduleArgs {
     unsigned long long *visits;          // lineages the scheduled rounds process
     unsigned int *n_resident;            // active simulations owned by the resident kernel
     unsigned int *blocks_done;           // the next round's kernel arrivals (reset here)
-    unsigned long long *rounds_seen;     // the most rounds that a simulation has begun
+    unsigned long long *rounds_seen;     // the most rounds scheduled for a simulation here (SimCounters.n_scheduled)
 };
 
 // the step kernel on grid x block and, with a.coop_max > 0, the cooperative
@@ -132,7 +132,6 @@ struct ResidentArgs {
     unsigned long long *steps_total;
     unsigned long long *visits;
     unsigned int *n_resident;
-    unsigned long long *rounds_seen;     // the most rounds that a simulation has begun
     const int *stop_flag;                // set when the concurrent global rounds end (nullable)
     uint32_t exp_sampler;                // 1: exponential event-time sampler (exp.rs), else Poisson
     const SmGate *gate;                  // SM reservation (nullable) and this engine's role in it

@@ -154,6 +154,7 @@ struct SimCounters {
     unsigned long long n_speciation;
     unsigned long long n_dedup;
     unsigned long long n_rounds;
+    unsigned long long n_scheduled;    // of these, begun by the schedule kernel
     unsigned long long n_live;         // live lineages at the round start
     unsigned long long n_live_next;    // survivors of the current round
     unsigned long long n_dispersal;
