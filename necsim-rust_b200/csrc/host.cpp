@@ -24,6 +24,7 @@
 #include "kernels.h"
 #include "layout.h"
 #include "tables.h"
+#include "workspace_pool.h"
 #include "wrapping_noise.h"
 
 using namespace necsim;
@@ -664,7 +665,7 @@ struct Control {  // small device scalars
 };
 
 // Host memory for events, grown on demand and not zeroed.  Kept between calls
-// (up to EnginePool::kHostBytes): the page faults of fresh memory made 34 MB of
+// (up to kKeptHostBytes): the page faults of fresh memory made 34 MB of
 // records take 14 ms to copy from the device instead of 1.5 ms.
 struct HostBuffer {
     std::unique_ptr<unsigned char[]> data;
@@ -780,6 +781,9 @@ struct Engine {
     ~Engine() { release(); }
 
     size_t bytes() const { return arena_bytes + sort_bytes; }
+    void drop_host_memory() {
+        for (auto &h : host_events) h = HostBuffer();
+    }
 
     // Frees what a run's origins were described with.
     void drop_inputs() {
@@ -806,7 +810,7 @@ struct Engine {
         if (sort_mem) cudaFree(sort_mem);
         arena = sort_mem = nullptr;
         arena_bytes = sort_bytes = 0;
-        for (auto &h : host_events) h = HostBuffer();
+        drop_host_memory();
         drop_inputs();
         for (auto p : d_cells)
             if (p) cudaFree(p);
@@ -2107,112 +2111,67 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
 // device, scenario kind and launch arguments, at most as many lineages):
 // setting them up and freeing them took 6 ms (a call with 1,200 lineages 7.5
 // ms, now 0.6 ms; with 100,000 lineages 11 ms, now 4.0 ms).  An
-// engine is in the pool only while no call uses it; the pool holds at most
-// kEngines engines and 1/32 of a device's memory each way, and is emptied
-// when an allocation fails.  Nothing in it depends on a call's inputs: every
+// engine is in the pool (workspace_pool.h) only while no call uses it; the
+// pool holds at most four engines and 1/32 of a device's memory, and is
+// emptied when an allocation fails.  Nothing in it depends on a call's inputs: every
 // run writes its lineages, parameters and counters anew.
-struct EnginePool {
-    static constexpr size_t kEngines = 4;
-    static constexpr size_t kHostBytes = 64 << 20;  // per host buffer of an idle engine
-    std::mutex mu;
-    std::vector<std::unique_ptr<Engine>> idle;
+constexpr size_t kKeptHostBytes = 64 << 20;  // per host buffer of an idle engine
 
-    // The id of the current CUDA context (0: unknown): engines of a context
-    // that the program has reset since are forgotten, not freed.
-    static unsigned long long context_id() {
-        using GetId = int (*)(void *, unsigned long long *);
-        static const GetId get = [] {
-            void *fn = nullptr;
-            cudaDriverEntryPointQueryResult q;
-            if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-                q != cudaDriverEntryPointSuccess) {
-                cudaGetLastError();
-                fn = nullptr;
-            }
-            return reinterpret_cast<GetId>(fn);
-        }();
+// The ids of the devices' CUDA contexts (0: none, or unknown).
+struct CudaContexts {
+    template <typename Fn>
+    static Fn entry(const char *name, unsigned version) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion(name, &fn, version, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<Fn>(fn);
+    }
+
+    static unsigned long long of(int device) {
+        static const auto get_id = entry<int (*)(void *, unsigned long long *)>("cuCtxGetId", 12000);
+        static const auto get_state = entry<int (*)(int, unsigned *, int *)>("cuDevicePrimaryCtxGetState", 7000);
+        unsigned flags = 0;
+        int active = 0, before = 0;
+        // (making a device current gives it a context)
+        if (!get_id || !get_state || get_state(device, &flags, &active) != 0 || !active) return 0;
+        if (cudaGetDevice(&before) != cudaSuccess || (before != device && cudaSetDevice(device) != cudaSuccess)) {
+            cudaGetLastError();
+            return 0;
+        }
         unsigned long long id = 0;
-        return get && get(nullptr, &id) == 0 ? id : 0;
-    }
-
-    static size_t byte_limit(int device) {
-        static std::mutex m;
-        static std::map<int, size_t> limits;
-        std::lock_guard<std::mutex> lock(m);
-        auto it = limits.find(device);
-        if (it == limits.end()) {
-            cudaDeviceProp prop;
-            CK(cudaGetDeviceProperties(&prop, device));
-            it = limits.emplace(device, prop.totalGlobalMem / 32).first;
-        }
-        return it->second;
-    }
-
-    // Arguments that an engine's buffers, launch shapes and graph depend on.
-    static bool same_shape(const Engine &E, int kind, const necsim_args &a) {
-        const necsim_args &b = E.args;
-        return E.kind == kind && a.device == E.device && a.block_size == b.block_size &&
-               a.grid_size == b.grid_size && a.dedup_factor_pct == b.dedup_factor_pct &&
-               a.rounds_per_graph == b.rounds_per_graph && a.report_dispersal == b.report_dispersal &&
-               a.event_time_sampler == b.event_time_sampler && a.schedule == 0 && b.schedule == 0;
-    }
-
-    // An idle engine with room for n lineages and disp dispersal events (the
-    // smallest one; not one with more than 8 times the room, whose buffers
-    // would be spread over memory for nothing), or null.
-    std::unique_ptr<Engine> take(int kind, const necsim_args &a, uint64_t n, uint64_t disp) {
-        const unsigned long long id = context_id();
-        std::lock_guard<std::mutex> lock(mu);
-        size_t best = idle.size();
-        for (size_t j = 0; j < idle.size(); ++j) {
-            const Engine &E = *idle[j];
-            if (id == 0 || E.context != id || !same_shape(E, kind, a) || E.n_cap < n || E.disp_room < disp) continue;
-            if (E.n_cap > 8 * std::max<uint64_t>(n, 4096)) continue;
-            if (best == idle.size() || E.n_cap < idle[best]->n_cap) best = j;
-        }
-        if (best == idle.size()) return nullptr;
-        std::unique_ptr<Engine> e = std::move(idle[best]);
-        idle.erase(idle.begin() + (std::ptrdiff_t)best);
-        return e;
-    }
-
-    void put(std::unique_ptr<Engine> e) {
-        const unsigned long long id = context_id();
-        const size_t limit = byte_limit(e->device);
-        if (id == 0 || e->args.schedule || e->bytes() > limit) return;
-        e->context = id;
-        for (auto &h : e->host_events)
-            if (h.bytes > kHostBytes) h = HostBuffer();
-        std::vector<std::unique_ptr<Engine>> gone;  // freed after the lock
-        std::lock_guard<std::mutex> lock(mu);
-        for (size_t j = 0; j < idle.size();) {
-            if (idle[j]->device == e->device && idle[j]->context != id) {
-                (void)idle[j].release();  // its context is gone, and its memory with it
-                idle.erase(idle.begin() + (std::ptrdiff_t)j);
-            } else {
-                ++j;
-            }
-        }
-        size_t bytes = e->bytes();
-        for (auto &o : idle) bytes += o->device == e->device ? o->bytes() : 0;
-        // the longest idle go first
-        while (!idle.empty() && (idle.size() >= kEngines || bytes > limit)) {
-            if (idle.front()->device == e->device) bytes -= idle.front()->bytes();
-            gone.push_back(std::move(idle.front()));
-            idle.erase(idle.begin());
-        }
-        idle.push_back(std::move(e));
-    }
-
-    bool empty_out() {
-        std::vector<std::unique_ptr<Engine>> gone;
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            gone.swap(idle);
-        }
-        return !gone.empty();
+        if (get_id(nullptr, &id) != 0) id = 0;
+        if (before != device) cudaSetDevice(before);
+        return id;
     }
 };
+
+using EnginePool = WorkspacePool<Engine, CudaContexts>;
+
+size_t workspace_limit(int device) {
+    static std::mutex m;
+    static std::map<int, size_t> limits;
+    std::lock_guard<std::mutex> lock(m);
+    auto it = limits.find(device);
+    if (it == limits.end()) {
+        cudaDeviceProp prop;
+        CK(cudaGetDeviceProperties(&prop, device));
+        it = limits.emplace(device, prop.totalGlobalMem / 32).first;
+    }
+    return it->second;
+}
+
+// Whether an engine's buffers, launch shapes and graph are those of the arguments.
+bool same_shape(const Engine &E, int kind, const necsim_args &a) {
+    const necsim_args &b = E.args;
+    return E.kind == kind && a.device == E.device && a.block_size == b.block_size && a.grid_size == b.grid_size &&
+           a.dedup_factor_pct == b.dedup_factor_pct && a.rounds_per_graph == b.rounds_per_graph &&
+           a.report_dispersal == b.report_dispersal && a.event_time_sampler == b.event_time_sampler &&
+           a.schedule == 0 && b.schedule == 0;
+}
 
 // Never destroyed: at process exit the CUDA context may be gone first.
 EnginePool &engine_pool() {
@@ -2221,6 +2180,25 @@ EnginePool &engine_pool() {
 }
 
 bool release_idle_workspaces() { return engine_pool().empty_out(); }
+
+// An idle engine with room for n lineages and disp dispersal events (the
+// smallest one; not one with more than 8 times the room, whose buffers would
+// be spread over memory for nothing), or null.
+std::unique_ptr<Engine> take_engine(int kind, const necsim_args &a, uint64_t n, uint64_t disp) {
+    return engine_pool().take(a.device, [&](const Engine &E) -> unsigned long long {
+        if (!same_shape(E, kind, a) || E.n_cap < n || E.disp_room < disp) return 0;
+        if (E.n_cap > 8 * std::max<uint64_t>(n, 4096)) return 0;
+        return E.n_cap + 1;
+    });
+}
+
+void keep_engine(std::unique_ptr<Engine> e) {
+    if (e->args.schedule) return;
+    for (auto &h : e->host_events)
+        if (h.bytes > kKeptHostBytes) h = HostBuffer();
+    const size_t limit = workspace_limit(e->device);
+    engine_pool().put(std::move(e), limit);
+}
 
 // ---- a batch split into engines: priority simulations each run alone ----
 //
@@ -2600,7 +2578,7 @@ static int simulate_impl(necsim_ctx *ctx, const necsim_lineage *lineages, uint64
         // (WrappingNoise counts its origins on the device: any engine may turn
         // out too small, then it gets buffers of its own)
         std::unique_ptr<Engine> E =
-            engine_pool().take(device_kind(sh.sc.kind), ctx->args, sh.n_origins, dispersal_room(ctx->args, sims));
+            take_engine(device_kind(sh.sc.kind), ctx->args, sh.n_origins, dispersal_room(ctx->args, sims));
         if (!E) {
             E.reset(new Engine());
             setup_engine(*E, ctx->args);
@@ -2610,7 +2588,7 @@ static int simulate_impl(necsim_ctx *ctx, const necsim_lineage *lineages, uint64
                         ctx->remaining, ctx->tables_ready ? &prebuilt : nullptr);
         *outcome = o;
         E->drop_inputs();
-        engine_pool().put(std::move(E));
+        keep_engine(std::move(E));
     });
 }
 
