@@ -951,8 +951,15 @@ void choose_launch(Engine &E) {
     // / 32 / 64 / 128 / 256 events per launch: 583 / 540 / 511 / 519 / 518
     // ms, with the learned schedule 526 / 509 / 475 / 478 / 487 and 489 / 522
     // / 495 / 474 / 460 (two seeds).  Traces and dispersal events are
-    // collected round by round.
-    if (E.sims.size() > 1 && !E.tracing && !E.args.report_dispersal) E.slice = 128;
+    // collected round by round.  Not where warps step SpatiallyExplicit lineages
+    // event by event (select_run): two and four simulations on maps of 16 cells
+    // squared with delta_t 3 take 4.12 and 8.49 ms unsliced, 5.75 and 10.1 ms
+    // sliced.
+    bool by_event = false;
+    for (const SimHost &sh : E.sims)
+        by_event |= E.kind == NECSIM_SPATIALLY_EXPLICIT && E.args.event_time_sampler != NECSIM_SAMPLER_EXP &&
+                    !(sh.params.chain & kChainPoisson);
+    if (E.sims.size() > 1 && !E.tracing && !E.args.report_dispersal && !by_event) E.slice = 128;
 }
 
 void carve_run_buffers(Engine &E, Carver &c) {

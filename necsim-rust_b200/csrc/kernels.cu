@@ -579,9 +579,10 @@ __device__ __forceinline__ bool noise_target_coop(const SimParams &p, const Nois
 // selection.  Side effects happen on lane 0 only; every lane returns with
 // the same updated lineage.  EXP selects the exponential event-time
 // sampler, searched by exp_search_coop.
+// With `quit` it stops before the event, with the peek kept.
 template <int KIND, bool EXP = false>
 __device__ __forceinline__ int lineage_step_coop(Lane &l, const SimParams &p, const EventSink &k,
-                                                 const NoiseLane &noise_lanes) {
+                                                 const NoiseLane &noise_lanes, bool quit = false) {
     const unsigned lane = threadIdx.x & 31u;
     const uint64_t loc_term = location_term(p.seed, lane_injection<KIND>(l, p));
     const PoissonConsts &pc = poisson_consts<KIND>(l, p);
@@ -680,7 +681,7 @@ __device__ __forceinline__ int lineage_step_coop(Lane &l, const SimParams &p, co
         e3 = __shfl_sync(kFull, dk, 2);
         e4 = __shfl_sync(kFull, dk, 3);
     }
-    if (__double_as_longlong(l.next) >= __double_as_longlong(l.horizon)) return kStepStop;
+    if (quit || __double_as_longlong(l.next) >= __double_as_longlong(l.horizon)) return kStepStop;
     if constexpr (KIND == kWrappingNoise) {
         // lineage_event, with the target found by the whole warp
         l.steps += 1;
@@ -1489,14 +1490,35 @@ __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const Even
     return result;
 }
 
-// A lineage's round by one warp: chain_run where it applies, else coop_run.
+// A lineage's round by one warp, event by event (lineage_step_coop).
+template <int KIND>
+__device__ __forceinline__ int select_run(Lane &l, const SimParams &p, const EventSink &k, uint64_t &events,
+                                          const NoiseLane &noise_lanes, const volatile unsigned *stop) {
+    for (;;) {
+        const bool quit = stop && (events & 31u) == 0u &&
+                          __shfl_sync(kFull, (threadIdx.x & 31u) == 0u ? *stop : 1u, 0) == 0u;
+        const int r = lineage_step_coop<KIND>(l, p, k, noise_lanes, quit);
+        if (r == kStepMoved || r == kStepSpeciated) events += 1;
+        if (r != kStepMoved) return r;
+    }
+}
+
+// A lineage's round by one warp: chain_run where it applies, else coop_run or
+// select_run.  A WrappingNoise target takes the whole warp.  SpatiallyExplicit
+// (a delta_t that is no power of two): the alias and record reads of coop_run's
+// speculative candidates cost more than they save: maps of 64 and 90 cells
+// squared with delta_t 3 take 13.8 and 14.4 ms with coop_run, 11.1 and 12.4 ms
+// with select_run.
 template <int KIND>
 __device__ __forceinline__ int warp_run(Lane &l, const SimParams &p, const EventSink &k, uint64_t &events,
-                                        const volatile unsigned *stop = nullptr) {
+                                        const NoiseLane &noise_lanes, const volatile unsigned *stop = nullptr) {
     if constexpr (kChainKind<KIND>) {
         if (chain_takes<KIND, false>(p, l)) return chain_run<KIND, false>(l, p, k, events, stop);
     }
-    return coop_run<KIND>(l, p, k, events, stop);
+    if constexpr (KIND == kWrappingNoise || KIND == kSpatiallyExplicit)
+        return select_run<KIND>(l, p, k, events, noise_lanes, stop);
+    else
+        return coop_run<KIND>(l, p, k, events, stop);
 }
 
 __device__ __forceinline__ EventSink sink_of(const StepArgs &a) {
@@ -1740,19 +1762,7 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
             }
             if (!chain && r == kStepSpeciated) warp_steps += 1;
         } else {
-            if constexpr (!kChainKind<KIND>) {
-                // the speculative candidates' alias and record reads cost more
-                // than they save here: select first, then read (measured); a
-                // noise target takes the whole warp
-                for (;;) {
-                    r = lineage_step_coop<KIND, false>(c, p, sink, noise_lanes);
-                    if (r != kStepMoved) break;
-                    warp_steps += 1;
-                }
-                if (r == kStepSpeciated) warp_steps += 1;
-            } else {
-                r = warp_run<KIND>(c, p, sink, warp_steps);
-            }
+            r = warp_run<KIND>(c, p, sink, warp_steps, noise_lanes);
             // the lineage's own round is done: it no longer holds the launch
             if (a.busy && lane_id == 0) atomicSub(a.busy, 1u);
             // A simulation that started the round with one live lineage has
@@ -1777,7 +1787,7 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
                     __syncwarp();
                     c.horizon = h;
                     // interrupted at a peek once the launch's regular work is done
-                    r = warp_run<KIND>(c, p, sink, warp_steps, SINGLE ? nullptr : a.busy);
+                    r = warp_run<KIND>(c, p, sink, warp_steps, noise_lanes, SINGLE ? nullptr : a.busy);
                     if (r == kStepStop && __double_as_longlong(c.next) < __double_as_longlong(h)) {
                         // the round is not finished: give it back, so the
                         // scheduler sets (and counts) the same horizon again
@@ -2064,7 +2074,7 @@ __global__ void __launch_bounds__(THREADS, 1) resident_kernel(ResidentArgs a) {
                         }
                     } else {
                         uint64_t ev = 0;
-                        c_live = warp_run<KIND>(c, p, sink, ev) == kStepStop;
+                        c_live = warp_run<KIND>(c, p, sink, ev, NoiseLane{}) == kStepStop;
                         my_events += ev;
                     }
                     if ((t & 31u) == 0) {
