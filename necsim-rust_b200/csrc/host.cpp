@@ -937,9 +937,7 @@ void choose_launch(Engine &E) {
         CK(coop_kernel_occupancy(E.kind, E.args.event_time_sampler == NECSIM_SAMPLER_EXP, &coop_per_sm));
         if (coop_per_sm < 1) coop_per_sm = 1;
         E.coop_grid = (unsigned)(coop_per_sm * E.n_sms);
-        E.coop_max = (uint64_t)E.coop_grid * (kCoopBlock / 32) * 4;
-        // a noise target takes a whole warp: every WrappingNoise round
-        if (E.kind == NECSIM_WRAPPING_NOISE) E.coop_max = ~0ULL;
+        E.coop_max = (uint64_t)E.coop_grid * (kCoopBlock / 32) * 4;  // (WrappingNoise: noise_coop_max)
     }
     E.aux_block = 256;
     E.aux_grid = (unsigned)(E.n_sms * 8);
@@ -951,15 +949,40 @@ void choose_launch(Engine &E) {
     // / 32 / 64 / 128 / 256 events per launch: 583 / 540 / 511 / 519 / 518
     // ms, with the learned schedule 526 / 509 / 475 / 478 / 487 and 489 / 522
     // / 495 / 474 / 460 (two seeds).  Traces and dispersal events are
-    // collected round by round.  Not where warps step SpatiallyExplicit lineages
-    // event by event (select_run): two and four simulations on maps of 16 cells
+    // collected round by round.  Not for WrappingNoise, nor where warps step
+    // SpatiallyExplicit lineages event by event (select_run): two and four simulations on maps of 16 cells
     // squared with delta_t 3 take 4.12 and 8.49 ms unsliced, 5.75 and 10.1 ms
     // sliced.
-    bool by_event = false;
+    bool by_event = E.kind == NECSIM_WRAPPING_NOISE;
     for (const SimHost &sh : E.sims)
         by_event |= E.kind == NECSIM_SPATIALLY_EXPLICIT && E.args.event_time_sampler != NECSIM_SAMPLER_EXP &&
                     !(sh.params.chain & kChainPoisson);
     if (E.sims.size() > 1 && !E.tracing && !E.args.report_dispersal && !by_event) E.slice = 128;
+}
+
+// WrappingNoise: rounds of at most this many live lineages give each a warp,
+// which evaluates its targets' octaves side by side; the step kernel gives it
+// a lane, which evaluates `octaves` for each of about 1 / coverage targets one
+// after the other (e evaluations per event; none at coverage 0 or 1).  A warp's
+// event takes the same time whatever e, a lane's grows with it, and lanes need
+// many lineages to fill the device.  One round (ms, lane / warp, Poisson):
+//   lineages    4,000       16,000      64,000      256,000     1,000,000
+//   e = 1.1     3.0 / 2.5   1.0 / 2.1   0.5 / 2.4   0.7 / 6.3   2.2 / 23.8
+//   e = 4       6.9 / 2.2   2.2 / 2.0   1.0 / 2.3   1.5 / 6.1   5.2 / 22.9
+//   e = 10     16.6 / 2.2   5.2 / 1.9   2.1 / 2.2   3.1 / 5.9  10.7 / 22.3
+//   e = 32     46.0 / 2.4  14.5 / 2.1   7.2 / 2.4   9.5 / 6.3  31.2 / 23.8
+// The exponential sampler's warps take 3.0 ms at 4,000 to 64,000 lineages and
+// 33 ms at 1,000,000 (e = 32: lane 29.8, 9.7, 5.3, 6.8 and 17.0 ms).
+uint64_t noise_coop_max(const std::vector<SimHost> &sims, bool exp_sampler) {
+    double e = 0.0, weight = 0.0;
+    for (const SimHost &sh : sims) {
+        const double c = sh.sc.coverage, n = (double)std::max<uint64_t>(sh.n_origins, 1);
+        e += n * std::max(1.0, c > 0.0 && c < 1.0 ? (double)sh.sc.octaves / c : 0.0);
+        weight += n;
+    }
+    e /= weight;
+    if (exp_sampler) return e > 48.0 ? ~0ULL : (uint64_t)std::max(4500.0, 1800.0 * e * std::max(1.0, e / 16.0));
+    return e > 24.0 ? ~0ULL : (uint64_t)std::max(5000.0, 4500.0 * e * std::max(1.0, e / 10.0));
 }
 
 void carve_run_buffers(Engine &E, Carver &c) {
@@ -2106,6 +2129,15 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
         }
         alloc_run_buffers(E, n_cap);
         create_round_events(E);
+    }
+    if (E.kind == NECSIM_WRAPPING_NOISE) {
+        // (a kept workspace's graph has its own run's limit)
+        const uint64_t most = noise_coop_max(E.sims, E.args.event_time_sampler == NECSIM_SAMPLER_EXP);
+        if (most != E.coop_max && E.graph_exec) {
+            CK(cudaGraphExecDestroy(E.graph_exec));
+            E.graph_exec = nullptr;
+        }
+        E.coop_max = most;
     }
     upload_origins(E, given);
     if (E.n_total > 0 && !E.lazy_graph) build_graph(E);

@@ -2464,18 +2464,15 @@ static cudaError_t launch_step_t(const StepArgs &a, unsigned grid, unsigned bloc
         else
             launch_coop_t<KIND, false>(a, coop_grid, st);
     }
-    // (a WrappingNoise target takes a whole warp: every round is cooperative)
-    if constexpr (KIND != kWrappingNoise) {
-        if (a.exp_sampler) {
-            if (a.n_sims == 1)
-                step_kernel_exp<KIND, true><<<grid, block, 0, st>>>(a);
-            else
-                step_kernel_exp<KIND, false><<<grid, block, 0, st>>>(a);
-        } else if (a.n_sims == 1) {
-            step_kernel<KIND, true><<<grid, block, 0, st>>>(a);
-        } else {
-            step_kernel<KIND, false><<<grid, block, 0, st>>>(a);
-        }
+    if (a.exp_sampler) {
+        if (a.n_sims == 1)
+            step_kernel_exp<KIND, true><<<grid, block, 0, st>>>(a);
+        else
+            step_kernel_exp<KIND, false><<<grid, block, 0, st>>>(a);
+    } else if (a.n_sims == 1) {
+        step_kernel<KIND, true><<<grid, block, 0, st>>>(a);
+    } else {
+        step_kernel<KIND, false><<<grid, block, 0, st>>>(a);
     }
     return cudaGetLastError();
 }
@@ -2513,13 +2510,9 @@ cudaError_t coop_kernel_occupancy(int kind, bool exp_sampler, int *blocks_per_sm
 
 template <int KIND>
 static cudaError_t step_occupancy_t(bool exp_sampler, int block, int *blocks_per_sm) {
-    if constexpr (KIND == kWrappingNoise) {  // (no step kernel)
-        return coop_occupancy_t<KIND>(exp_sampler, blocks_per_sm);
-    } else {
-        if (exp_sampler)
-            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel_exp<KIND, false>, block, 0);
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<KIND, false>, block, 0);
-    }
+    if (exp_sampler)
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel_exp<KIND, false>, block, 0);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<KIND, false>, block, 0);
 }
 
 cudaError_t step_kernel_occupancy(int kind, bool exp_sampler, int block, int *blocks_per_sm) {

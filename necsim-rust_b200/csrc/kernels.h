@@ -51,8 +51,8 @@ struct StepArgs {
     uint32_t n_sims;                     // simulations in `params`
     TraceSink trace;                     // death records of speciated lineages (tracing only)
     uint32_t exp_sampler;                // 1: exponential event-time sampler (exp.rs), else Poisson
-    // rounds with at most this many live lineages run in the cooperative kernel (one warp per lineage); 0: the step kernel takes
-    // every round (WrappingNoise: ~0, it takes none)
+    // rounds with at most this many live lineages run in the cooperative
+    // kernel (one warp per lineage); 0: the step kernel takes every round
     uint64_t coop_max;
     uint32_t n_sms;                      // SMs the kernels' grids are spread over
     // Batches: the step kernel runs at most this many events of a lineage in
@@ -109,8 +109,7 @@ struct ScheduleArgs {
 };
 
 // the step kernel on grid x block and, with a.coop_max > 0, the cooperative
-// kernel on coop_grid x kCoopBlock before it
-// (WrappingNoise: every round runs there); each returns at once in the
+// kernel on coop_grid x kCoopBlock before it; each returns at once in the
 // other's rounds
 cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned block, unsigned coop_grid,
                         cudaStream_t st);
