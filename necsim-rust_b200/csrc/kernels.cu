@@ -2464,6 +2464,7 @@ static cudaError_t launch_step_t(const StepArgs &a, unsigned grid, unsigned bloc
         else
             launch_coop_t<KIND, false>(a, coop_grid, st);
     }
+    if (grid == 0) return cudaGetLastError();
     if (a.exp_sampler) {
         if (a.n_sims == 1)
             step_kernel_exp<KIND, true><<<grid, block, 0, st>>>(a);

@@ -110,7 +110,7 @@ struct ScheduleArgs {
 
 // the step kernel on grid x block and, with a.coop_max > 0, the cooperative
 // kernel on coop_grid x kCoopBlock before it; each returns at once in the
-// other's rounds
+// other's rounds (grid 0: no round is the step kernel's)
 cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned block, unsigned coop_grid,
                         cudaStream_t st);
 cudaError_t step_kernel_occupancy(int kind, bool exp_sampler, int block, int *blocks_per_sm);
