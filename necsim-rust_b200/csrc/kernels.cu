@@ -1478,14 +1478,16 @@ __device__ __forceinline__ int chain_run(Lane &l, const SimParams &p, const Even
     else if (result == kStepMoved)
         result = chain_phase<KIND, KIND != kSpatiallyImplicit, EXP>(c, l, p, k, stop);
     l.steps += c.moved;
-    if (l.steps != steps) l.last = EXP ? c.before : __dmul_rn(c.before, p.delta_t);
+    if (l.steps != steps) {  // (else it is where it was)
+        l.last = EXP ? c.before : __dmul_rn(c.before, p.delta_t);
+        chain_unpack<KIND>(p, c.loc_term, c.local, c.cell, l.x, l.y, l.i);
+        if (KIND == kSpatiallyExplicit) l.rec = c.rec;
+    }
     if (result == kStepSpeciated) l.steps += 1;
     events += l.steps - steps;
     l.next = EXP ? c.next : __dmul_rn(c.next, p.delta_t);
     l.reprime = c.reprime;
     l.has_next = result == kStepStop;
-    chain_unpack<KIND>(p, c.loc_term, c.local, c.cell, l.x, l.y, l.i);
-    if (KIND == kSpatiallyExplicit) l.rec = c.rec;
     if (result == kStepSpeciated && (threadIdx.x & 31u) == 0u) emit_speciation(l, k);
     return result;
 }
