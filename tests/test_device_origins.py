@@ -63,3 +63,16 @@ def test_batch_segments(nb, syn):
     for a, b in zip(one, many):
         assert np.array_equal(a.speciation, b.speciation)
         assert (a.n_initial, a.steps) == (b.n_initial, b.steps)
+
+
+def test_batch_of_noise(nb, syn):
+    """Many small samples, some of them without a habitable location."""
+    scenarios = [syn.to_scenario(noise((0.0, 0.4, 1.0, 0.7)[s % 4], (M32 - 3 + 5 * s, 7 * s, 1 + s % 5, 1 + s % 9)))
+                 for s in range(61)]
+    got = nb.simulate_batch(scenarios, [0.05] * 61, list(range(61)), nb.CUDA(), collect=True)
+    assert [g.n_initial for g in got] == [len(nb.enumerate_origins(s)) for s in scenarios]
+    for s in (0, 1, 2, 3, 31, 58, 59, 60):
+        one = nb.simulate(0.05, scenarios[s], s)
+        assert np.array_equal(one.speciation, got[s].speciation) and one.steps == got[s].steps
+    none = nb.simulate_batch(scenarios[:61:4], [0.05] * 16, list(range(16)), nb.CUDA(), collect=True)
+    assert all((g.n_initial, g.steps) == (0, 0) for g in none)
