@@ -76,3 +76,25 @@ def test_batch_of_noise(nb, syn):
         assert np.array_equal(one.speciation, got[s].speciation) and one.steps == got[s].steps
     none = nb.simulate_batch(scenarios[:61:4], [0.05] * 16, list(range(16)), nb.CUDA(), collect=True)
     assert all((g.n_initial, g.steps) == (0, 0) for g in none)
+
+
+@pytest.mark.parametrize("kind", ["circles", "maps"])
+def test_batch_of_prefix_sums(nb, syn, kind):
+    """Circles of many radii beside rectangles, and maps of many shapes: each
+    simulation reads its own part of the batch's prefix sums."""
+    if kind == "circles":
+        descs = [dict(kind=2, sigma=2.0, radius=s % 7, centre_x=3 * s, centre_y=M32 - s) if s % 5 else
+                 dict(kind=2, sigma=2.0, sample=(s, s, 1 + s, 2)) for s in range(23)]
+    else:
+        descs = []
+        for s in range(9):
+            hab = syn.habitat_map(1 + 2 * s, 1 + s % 4, 0.4, 5, 11 + s)
+            hab.flat[0] = 1
+            descs.append(dict(kind=3, width=hab.shape[1], height=hab.shape[0], habitat=hab,
+                              dispersal=syn.dispersal_map(hab, 1.5)))
+    scenarios = [syn.to_scenario(d) for d in descs]
+    got = nb.simulate_batch(scenarios, [0.05] * len(descs), list(range(len(descs))), nb.CUDA(), collect=True)
+    for s, g in enumerate(got):
+        one = nb.simulate(0.05, scenarios[s], s)
+        assert np.array_equal(one.speciation, g.speciation) and one.steps == g.steps
+        assert g.n_initial == len(nb.enumerate_origins(scenarios[s]))
