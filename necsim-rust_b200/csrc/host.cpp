@@ -738,7 +738,7 @@ struct Engine {
     Control *h_ctl = nullptr;  // pinned
 
     unsigned step_grid = 0, step_block = 0;
-    unsigned coop_grid = 0;   // cooperative kernel (Poisson sampler), kCoopBlock threads per block
+    unsigned coop_grid = 0;   // cooperative kernel, kCoopBlock threads per block
     uint64_t coop_max = 0;    // rounds with at most this many live lineages run there
     unsigned aux_grid = 0, aux_block = 256;
     uint32_t slice = 0;  // events of a lineage per launch of the step kernel (StepArgs)
@@ -927,7 +927,7 @@ void choose_launch(Engine &E) {
         // One warp per lineage, for rounds of up to four lineages per
         // resident warp (9,472 with four blocks per SM).  The cooperative
         // kernel steps about 4e9 events per second whatever the round's size
-        // (329 warp instructions per event), the step kernel, one lane per
+        // (258 warp instructions per event), the step kernel, one lane per
         // lineage, 7e9 with 30,000 live lineages of one simulation and 2 to
         // 3e9 with 20,000 to 50,000 of many.  A limit of one / two / four /
         // eight lineages per warp: the 64-simulation sweep takes 637 / 593 /
@@ -1326,8 +1326,7 @@ FeatureArgs make_feature_args(Engine &E, DeviceLineages &in) {
     f.params = E.d_params;
     f.counters = E.d_counters;
     f.kind = E.kind;
-    // rounds stepped one warp at a time per lineage (the cooperative kernel, or the
-    // exponential sampler's step kernel when it has a warp per lineage)
+    // rounds that the cooperative kernel steps, a warp per lineage
     f.skip_at_most = E.coop_max;
     return f;
 }
@@ -2119,7 +2118,10 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
     if (off >= 0xffffffffULL) fail(NECSIM_E_TOO_LARGE, "more than 2^32 - 1 lineages");
     E.sims = std::move(sims);
     E.n_total = off;
-    // origins are numbered from 0 in every simulation; given lineages as they come
+    // Origins in cells are numbered from 0 in every simulation; given lineages
+    // come as they are.  (AlmostInfinite and WrappingNoise references are
+    // coordinates, (y << 32) | x: the device sorts by their low digits and the
+    // host settles the ties above.)
     E.references = 1;
     for (const SimHost &sh : E.sims) E.references = std::max<uint64_t>(E.references, sh.n_origins);
     if (given) E.references = 1ULL << 32;

@@ -129,8 +129,7 @@ __device__ __forceinline__ bool spatially_explicit_dispersal_draw(
 }  // namespace
 
 // Where an event left the lineage.
-// (kStepSlice: short of the horizon, the launch's events executed)
-enum StepResult : int { kStepStop = 0, kStepMoved = 1, kStepSpeciated = 2, kStepDropped = 3, kStepSlice = 5 };
+enum StepResult : int { kStepStop = 0, kStepMoved = 1, kStepSpeciated = 2, kStepDropped = 3 };
 
 // Outputs of lineage_step besides the lineage itself.
 struct EventSink {
@@ -965,12 +964,14 @@ __device__ __forceinline__ int coop_run(Lane &l, const SimParams &p, const Event
 //    Speciations, horizons, migrations and the rarer selections leave it
 //    with the event computed.
 // Measured with one lineage on a B200 (1,965 MHz), coop_run -> chain_run:
-// NonSpatial 1,772 -> 652 cycles per event, SpatiallyImplicit 1,747 -> 650,
-// AlmostInfinite Normal 2,793 -> 701, Clark2Dt 3,376 -> 725 (1,503 and 2,173
-// with f64 displacements), SpatiallyExplicit 3,020 -> 1,898 (64 x 64
-// map; its atoms, 193 MB, come from HBM).  The bound is the instruction count: a
-// lone warp issues one instruction every two cycles, and NonSpatial takes 329
-// per event (48 a prime, 31 a sample).
+// NonSpatial 1,770 -> 651 cycles per event, SpatiallyImplicit 1,745 -> 646,
+// AlmostInfinite Normal 2,790 -> 704, Clark2Dt 3,374 -> 715 (1,503 and 2,173
+// with f64 displacements), SpatiallyExplicit, which selected first
+// (lineage_step_coop), 2,776 -> 1,824 (64 x 64 map; its atoms, 193 MB, come
+// from HBM).  The bound is the latency of a lone warp's instructions: NonSpatial
+// takes 258 per event, each issued 2.5 cycles after the one before it (1.15 of
+// fixed latency, 0.24 dispatch, 0.21 and 0.10 short and long scoreboard, 0.11
+// missing instructions per issue).
 template <int KIND>
 constexpr bool kChainKind = KIND != kWrappingNoise;
 

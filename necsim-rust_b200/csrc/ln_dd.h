@@ -340,12 +340,13 @@ NECSIM_DD_FN double necsim_ln_full(double x) {
  * logarithm) from a shorter evaluation where that decides the rounding
  * (Ziv 1991), else from the full one.  With the same reduction,
  *   ln(1 + r) = r - r^2 / 2 + r^3 (1/3 - r/4 + ... + r^6/9):
- * r and r^2 / 2 enter exactly up to 2^-106, the cubic term in double: its
- * six roundings are 2^-50.4 of r^3 / 3 <= 2^-18.5 |r|, the series' end
- * 2^-79 |r|, the low words' sum 2^-53 of their largest, 2^-18.5 |r|; the
- * result is at least |r| / 4 (k ln 2 - ln c_i cancels at most that much), so
- * the relative error is below 2^-66.  One in about 2^12 inputs is evaluated
- * again.  About 60 operations instead of 150. */
+ * r and r^2 / 2 enter exactly up to 2^-106, the cubic term in double, at most
+ * 2^-18.5 |r|.  In units of 2^-53 of it: 4.5 for its products, coefficients
+ * and their constants, 3 for r's low word, which it leaves out, 2 for the low
+ * words' sum, whose largest it is: 2^-68.3 |r|.  The series' end is
+ * 2^-79 |r|.  The result is at least |r| / 4 (k ln 2 - ln c_i cancels at most
+ * that much), so the relative error is below 2^-66.  One in about 2^12 inputs
+ * is evaluated again.  About 60 operations instead of 150. */
 NECSIM_DD_FN double necsim_ln(double x) {
     uint64_t bits;
     double m, q, h2, l2, t, low, hi, lo, e;
