@@ -739,6 +739,7 @@ struct Engine {
 
     unsigned step_grid = 0, step_block = 0;
     unsigned coop_grid = 0;   // cooperative kernel, kCoopBlock threads per block
+    bool chain = false;       // some simulation may take the lone-lineage form (Poisson sampler)
     uint64_t coop_max = 0;    // rounds with at most this many live lineages run there
     unsigned aux_grid = 0, aux_block = 256;
     uint32_t slice = 0;  // events of a lineage per launch of the step kernel (StepArgs)
@@ -1301,6 +1302,7 @@ StepArgs make_step_args(Engine &E, DeviceLineages &in) {
     a.n_sims = (uint32_t)E.sims.size();
     a.order = E.learned ? E.order : nullptr;
     a.exp_sampler = E.args.event_time_sampler == NECSIM_SAMPLER_EXP ? 1u : 0u;
+    a.chain = E.chain ? 1u : 0u;
     a.coop_max = E.coop_max;
     a.slice = E.slice;
     a.n_sms = (uint32_t)E.n_sms;
@@ -2167,15 +2169,18 @@ void prepare_engine(Engine &E, std::vector<SimHost> sims, const necsim_args &arg
         alloc_run_buffers(E, n_cap);
         create_round_events(E);
     }
-    if (E.kind == NECSIM_WRAPPING_NOISE) {
-        // (a kept workspace's graph has its own run's limit)
-        const uint64_t most = noise_coop_max(E.sims, E.args.event_time_sampler == NECSIM_SAMPLER_EXP);
-        if (most != E.coop_max && E.graph_exec) {
-            CK(cudaGraphExecDestroy(E.graph_exec));
-            E.graph_exec = nullptr;
-        }
-        E.coop_max = most;
+    // (a kept workspace's graph has its own run's limit and kernels)
+    const uint64_t coop_max = E.kind == NECSIM_WRAPPING_NOISE
+                                  ? noise_coop_max(E.sims, E.args.event_time_sampler == NECSIM_SAMPLER_EXP)
+                                  : E.coop_max;
+    bool chain = false;
+    for (const SimHost &sh : E.sims) chain |= (sh.params.chain & kChainPoisson) != 0;
+    if (E.graph_exec && (coop_max != E.coop_max || chain != E.chain)) {
+        CK(cudaGraphExecDestroy(E.graph_exec));
+        E.graph_exec = nullptr;
     }
+    E.coop_max = coop_max;
+    E.chain = chain;
     upload_origins(E, given);
     if (E.n_total > 0 && !E.lazy_graph) build_graph(E);
 }

@@ -1511,11 +1511,11 @@ __device__ __forceinline__ int select_run(Lane &l, const SimParams &p, const Eve
 // (a delta_t that is no power of two): the alias and record reads of coop_run's
 // speculative candidates cost more than they save: maps of 64 and 90 cells
 // squared with delta_t 3 take 13.8 and 14.4 ms with coop_run, 11.1 and 12.4 ms
-// with select_run.
-template <int KIND>
+// with select_run.  CHAIN: chain_run is not ruled out.
+template <int KIND, bool CHAIN = true>
 __device__ __forceinline__ int warp_run(Lane &l, const SimParams &p, const EventSink &k, uint64_t &events,
                                         const NoiseLane &noise_lanes, const volatile unsigned *stop = nullptr) {
-    if constexpr (kChainKind<KIND>) {
+    if constexpr (CHAIN && kChainKind<KIND>) {
         if (chain_takes<KIND, false>(p, l)) return chain_run<KIND, false>(l, p, k, events, stop);
     }
     if constexpr (KIND == kWrappingNoise || KIND == kSpatiallyExplicit)
@@ -1732,7 +1732,7 @@ __device__ __forceinline__ void block_arrives(const SmGate *g, uint32_t role, un
 // steps each one with all its lanes (a lineage's events at warp latency,
 // lineages on all SMs).  At most a few lineages wait for each warp, so the
 // queue is not ordered (no order is computed for such rounds).
-template <int KIND, bool SINGLE, bool EXP>
+template <int KIND, bool SINGLE, bool EXP, bool CHAIN>
 __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P, uint64_t n) {
     const EventSink sink = sink_of(a);
     const unsigned lane_id = threadIdx.x & 31u;
@@ -1765,7 +1765,7 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
             }
             if (!chain && r == kStepSpeciated) warp_steps += 1;
         } else {
-            r = warp_run<KIND>(c, p, sink, warp_steps, noise_lanes);
+            r = warp_run<KIND, CHAIN>(c, p, sink, warp_steps, noise_lanes);
             // the lineage's own round is done: it no longer holds the launch
             if (a.busy && lane_id == 0) atomicSub(a.busy, 1u);
             // A simulation that started the round with one live lineage has
@@ -1790,7 +1790,7 @@ __device__ __forceinline__ void coop_body(const StepArgs &a, const SimParams *P,
                     __syncwarp();
                     c.horizon = h;
                     // interrupted at a peek once the launch's regular work is done
-                    r = warp_run<KIND>(c, p, sink, warp_steps, noise_lanes, SINGLE ? nullptr : a.busy);
+                    r = warp_run<KIND, CHAIN>(c, p, sink, warp_steps, noise_lanes, SINGLE ? nullptr : a.busy);
                     if (r == kStepStop && __double_as_longlong(c.next) < __double_as_longlong(h)) {
                         // the round is not finished: give it back, so the
                         // scheduler sets (and counts) the same horizon again
@@ -1933,7 +1933,12 @@ __global__ void __launch_bounds__(kStepBlockMax, 1) step_kernel_exp(StepArgs a) 
 // compiler keeps its chain within 128 registers, at 1,540 cycles per event
 // against 1,481 with 138 to 148; the Poisson sampler's 64-simulation sweep is
 // the slower one with more registers and fewer warps (494 -> 503 ms).
-template <int KIND, bool SINGLE, bool EXP>
+// CHAIN (Poisson sampler): some simulation's lineages may take chain_run.  A
+// kernel of their own for the runs without any: beside chain_run the general
+// forms of one NonSpatial and one SpatiallyImplicit lineage (delta_t 3) take
+// 2,032 and 2,038 cycles per event, AlmostInfinite 2,253, alone 2,009, 1,989 and
+// 2,125.
+template <int KIND, bool SINGLE, bool EXP, bool CHAIN>
 __global__ void __launch_bounds__(kCoopBlock, EXP ? 1 : 0) coop_kernel(StepArgs a) {
     __shared__ __align__(16) unsigned char params_smem[SINGLE ? sizeof(SimParams) : 16];
     const uint64_t n = *a.n_cur;
@@ -1942,7 +1947,7 @@ __global__ void __launch_bounds__(kCoopBlock, EXP ? 1 : 0) coop_kernel(StepArgs 
     if (a.gate_role == kGateNone && (uint64_t)blockIdx.x * warps >= n) return;
     if (block_leaves(a.gate, a.gate_role, a.blocks_done)) return;
     const SimParams *P = stage_params<SINGLE>(a, params_smem);
-    if (threadIdx.x / 32u < warps) coop_body<KIND, SINGLE, EXP>(a, P, n);
+    if (threadIdx.x / 32u < warps) coop_body<KIND, SINGLE, EXP, CHAIN>(a, P, n);
     block_arrives(a.gate, a.gate_role, a.blocks_done);
 }
 
@@ -2450,12 +2455,12 @@ __global__ void schedule_kernel(ScheduleArgs a) {
 }
 
 // ---- host-side launchers ----
-template <int KIND, bool EXP>
+template <int KIND, bool EXP, bool CHAIN>
 static void launch_coop_t(const StepArgs &a, unsigned coop_grid, cudaStream_t st) {
     if (a.n_sims == 1)
-        coop_kernel<KIND, true, EXP><<<coop_grid, kCoopBlock, 0, st>>>(a);
+        coop_kernel<KIND, true, EXP, CHAIN><<<coop_grid, kCoopBlock, 0, st>>>(a);
     else
-        coop_kernel<KIND, false, EXP><<<coop_grid, kCoopBlock, 0, st>>>(a);
+        coop_kernel<KIND, false, EXP, CHAIN><<<coop_grid, kCoopBlock, 0, st>>>(a);
 }
 
 template <int KIND>
@@ -2463,9 +2468,11 @@ static cudaError_t launch_step_t(const StepArgs &a, unsigned grid, unsigned bloc
                                  cudaStream_t st) {
     if (a.coop_max) {
         if (a.exp_sampler)
-            launch_coop_t<KIND, true>(a, coop_grid, st);
+            launch_coop_t<KIND, true, true>(a, coop_grid, st);
+        else if (kChainKind<KIND> && a.chain)
+            launch_coop_t<KIND, false, kChainKind<KIND>>(a, coop_grid, st);
         else
-            launch_coop_t<KIND, false>(a, coop_grid, st);
+            launch_coop_t<KIND, false, false>(a, coop_grid, st);
     }
     if (grid == 0) return cudaGetLastError();
     if (a.exp_sampler) {
@@ -2496,9 +2503,10 @@ cudaError_t launch_step(int kind, const StepArgs &a, unsigned grid, unsigned blo
 template <int KIND>
 static cudaError_t coop_occupancy_t(bool exp_sampler, int *blocks_per_sm) {
     if (exp_sampler)
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, coop_kernel<KIND, false, true>, kCoopBlock,
-                                                             0);
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, coop_kernel<KIND, false, false>, kCoopBlock, 0);
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, coop_kernel<KIND, false, true, true>,
+                                                             kCoopBlock, 0);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, coop_kernel<KIND, false, false, kChainKind<KIND>>,
+                                                         kCoopBlock, 0);
 }
 
 cudaError_t coop_kernel_occupancy(int kind, bool exp_sampler, int *blocks_per_sm) {

@@ -51,6 +51,7 @@ struct StepArgs {
     uint32_t n_sims;                     // simulations in `params`
     TraceSink trace;                     // death records of speciated lineages (tracing only)
     uint32_t exp_sampler;                // 1: exponential event-time sampler (exp.rs), else Poisson
+    uint32_t chain;                      // 1: some simulation may take the lone-lineage form (SimParams.chain)
     // rounds with at most this many live lineages run in the cooperative
     // kernel (one warp per lineage); 0: the step kernel takes every round
     uint64_t coop_max;

@@ -255,6 +255,7 @@ extern "C" int necsim_gpu_round_noalloc(const necsim_scenario *scenario, const n
     sa.n_sims = 1;
     sa.n_sms = sms;
     sa.exp_sampler = exp_sampler ? 1u : 0u;
+    sa.chain = p.chain & kChainPoisson ? 1u : 0u;
     sa.coop_max = (uint64_t)coop_grid * (kCoopBlock / 32) * 4;
     if (launch_step(scenario->kind, sa, step_grid, kBlock, coop_grid, st) != cudaSuccess) return NECSIM_E_CUDA;
 
