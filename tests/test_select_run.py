@@ -26,3 +26,22 @@ def test_matches_oracle(nb, syn, oracle, n_sims, resident, kw):
                             **dict(dict(step_slice=10, min_round_events=1 << 20, step_slice_max=1024), **kw))
         assert same_stream(g.speciation, c.speciation), s
         assert (g.steps, g.n_rounds, g.n_dedup, g.time) == (c.steps, c.n_rounds, c.n_dedup, c.time), s
+
+
+@pytest.mark.parametrize("kind", ["ns", "se"])
+def test_workspaces_across_delta_t(nb, syn, oracle, kind):
+    """Calls of hundreds of rounds with and without a lone-lineage form reuse
+    one another's workspace, whose graph holds the kernels of one of them."""
+    if kind == "ns":
+        desc = dict(kind=0, speciation_probability=2e-3, width=40, height=30, deme=2)
+    else:
+        desc = se(syn, 31, 29, 1.5, 2e-3, cell=3)
+    kw = dict(step_slice=1, min_round_events=1, step_slice_max=1)
+    want = {dt: oracle.simulate(desc, 5, mode=oracle.MODE_CANONICAL, delta_t=dt, **kw) for dt in (2.0, 3.0, 0.5)}
+    assert min(c.n_rounds for c in want.values()) > 500
+    for dt in (2.0, 3.0, 2.0, 0.5, 3.0, 3.0, 2.0):
+        g = nb.simulate(2e-3, syn.to_scenario(desc), 5, nb.CUDA(delta_t=dt, **kw))
+        c = want[dt]
+        assert g.n_step_launches > 300  # a graph was built
+        assert same_stream(g.speciation, c.speciation), dt
+        assert (g.steps, g.n_rounds, g.n_dedup, g.time) == (c.steps, c.n_rounds, c.n_dedup, c.time), dt
